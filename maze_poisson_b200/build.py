@@ -23,6 +23,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relax
 SOURCES = {
     "engine.cu": ["--fmad=false"],
     "cg_fast.cu": ["--fmad=false"],
+    "resident.cu": ["--fmad=false"],
     "particles.cu": ["--fmad=false"],
     "tf_forces.cu": ["--fmad=true"],
     "fft.cu": ["--fmad=false"],
@@ -32,7 +33,7 @@ SOURCES = {
     "pb.cu": ["--fmad=false"],
     "devmem.cu": ["--fmad=false"],
 }
-HEADERS = ["mzb_common.cuh", "engine.cuh", "particles.cuh", "fft.cuh", "tma.cuh", "mixed.cuh", "pb.cuh"]
+HEADERS = ["mzb_common.cuh", "engine.cuh", "particles.cuh", "fft.cuh", "tma.cuh", "mixed.cuh", "pb.cuh", "resident.cuh"]
 
 
 def _nvcc():

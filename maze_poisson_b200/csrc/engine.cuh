@@ -85,6 +85,9 @@ struct EngineArgs {
     // inverse of one 10^3 block's Laplacian (1000 x 1000, row-major), PC_BLOCKJACOBI
     const double* bj_inv;
 
+    // work area of the resident kernels (resident_halo_bytes(n)) or null: not used
+    void* halo;
+
     double* partials;  // 2 sets x 8 values x gridDim.x
     GridBarrier* bar;
     int* result;       // [0] program return value, [1] engine status (0 ok)

@@ -17,6 +17,7 @@
 #include "mixed.cuh"
 #include "particles.cuh"
 #include "pb.cuh"
+#include "resident.cuh"
 
 namespace mzb {
 
@@ -110,6 +111,7 @@ struct GridState {
     int nu1 = 3, nu2 = 2;
     double batch_cost = 1.0;  // batched-solve time per grid point relative to other sizes (mzb_batch_autotune)
     int lev_plan = -1;        // the plan the current levels were built for
+    void* halo = nullptr;      // work area of the resident CG kernel (ensure_halo)
     double* bj_inv = nullptr;  // block-Jacobi block inverse (1000 x 1000) on BLOCKJACOBI grids
     // Poisson-Boltzmann (solver_initialize_grid_pois_boltz, grid_general.c:84-100)
     bool pb = false;
@@ -175,6 +177,7 @@ void free_grid(GridState& G) {
     dfree(G.rc); dfree(G.ec); dfree(G.cr); dfree(G.cp0); dfree(G.cp1); dfree(G.cAp);
     G.fft.release();
     dfree(G.bj_inv);
+    dfree(G.halo);
     dfree(G.pbg.ex); dfree(G.pbg.ey); dfree(G.pbg.ez); dfree(G.pbg.k2); dfree(G.pbg.dg);
     dfree(G.pbg.cex); dfree(G.pbg.cey); dfree(G.pbg.cez); dfree(G.pbg.ck2); dfree(G.pbg.cdg);
     G.pbg = PbGrid{};
@@ -342,11 +345,20 @@ void set_pb_operator(EngineArgs& a, const PbGrid& g) {
     a.cex = g.cex; a.cey = g.cey; a.cez = g.cez; a.cdg = g.cdg;
 }
 
+// The resident CG kernel's work area, allocated at the first solve that can use it.
+void ensure_halo(GridState& G) {
+    if (G.halo) return;
+    const size_t bytes = resident_halo_bytes(G.n);
+    if (bytes) G.halo = dalloc<unsigned char>(bytes);
+}
+
 EngineArgs engine_base(System& s) {
     GridState& G = s.G;
+    if (G.type == G_LCG || G.type == G_MAZE_LCG) ensure_halo(G);
     EngineArgs a{};
     a.n = G.n;
     a.tol = G.tol;
+    a.halo = G.halo;
     a.r = G.r; a.p0 = G.p0; a.p1 = G.p1; a.Ap = G.Ap; a.v = G.v; a.rf = G.rf; a.tmp = G.tmp;
     a.rc = G.rc; a.ec = G.ec; a.cr = G.cr; a.cp0 = G.cp0; a.cp1 = G.cp1; a.cAp = G.cAp;
     a.partials = s.partials;
@@ -359,11 +371,18 @@ EngineArgs engine_base(System& s) {
     return a;
 }
 
+// Launch the solver for `a`: the resident kernel where its size and program allow, then the
+// TMA-staged CG, then the general engine (MZB_ENGINE=generic: always that).
+void launch_solver(const EngineArgs& a, cudaStream_t stream) {
+    static const bool generic_only = getenv("MZB_ENGINE") && strcmp(getenv("MZB_ENGINE"), "generic") == 0;
+    if (!generic_only && (resident_cg_launch(a, stream) || cg_fast_launch(a, stream))) return;
+    engine_launch(a, stream);
+}
+
 // Run the engine and return its result; an engine failure (a barrier that timed out)
 // is reported and turned into -1 ("not converged").
 int run_engine(System& s, const EngineArgs& a) {
     MZB_CHECK(cudaEventRecord(s.ev0, s.stream));
-    static const bool generic_only = getenv("MZB_ENGINE") && strcmp(getenv("MZB_ENGINE"), "generic") == 0;
     // MZB_PHASE_TIMING=1: time-stamp the phases of the CG kernel and print them (debug aid)
     static const bool stamps_on = getenv("MZB_PHASE_TIMING") != nullptr;
     static unsigned long long* stamps_d = nullptr;
@@ -373,7 +392,7 @@ int run_engine(System& s, const EngineArgs& a) {
         MZB_CHECK(cudaMemsetAsync(stamps_d, 0, sizeof(unsigned long long) * 96, s.stream));
         b.stamps = stamps_d;
     }
-    if (generic_only || !cg_fast_launch(b, s.stream)) engine_launch(a, s.stream);
+    launch_solver(b, s.stream);
     if (stamps_on) {
         unsigned long long h[96];
         MZB_CHECK(cudaMemcpyAsync(h, stamps_d, sizeof(h), cudaMemcpyDeviceToHost, s.stream));
@@ -1201,6 +1220,7 @@ EngineArgs scratch_engine(System& s, Work& w, int n) {
     a.tmp = w.get(m);
     a.rc = w.get(mc); a.ec = w.get(mc); a.cr = w.get(mc); a.cp0 = w.get(mc); a.cp1 = w.get(mc);
     a.cAp = w.get(mc);
+    if (const size_t bytes = resident_halo_bytes(n)) a.halo = w.get(bytes / sizeof(double));
     a.partials = s.partials;
     a.bar = s.bar;
     a.result = s.result;
@@ -1935,7 +1955,6 @@ int md_steps_deferred(System& s, int n_steps) {
     ParticleDev& P = s.P;
     batch_prepare(s);  // device charge total, error words, Philox counter
     double* bad = s.scratch_d + 4094;  // the last two words of the 4096-double scratch
-    static const bool generic_only = getenv("MZB_ENGINE") && strcmp(getenv("MZB_ENGINE"), "generic") == 0;
     for (int i = 0; i < n_steps; i++) {
         integrator_part1(P, s.I, s.stream);
         spread_charges(P, G.q, G.qmask, G.n, G.h, s.stream);
@@ -1951,8 +1970,7 @@ int md_steps_deferred(System& s, int n_steps) {
                 const int prog = mixed_update_prog(G, cst);
                 mixed_launch(mixed_args(s, prog, cst), s.stream);
             } else {
-                const EngineArgs a = update_engine_args(s);
-                if (generic_only || !cg_fast_launch(a, s.stream)) engine_launch(a, s.stream);
+                launch_solver(update_engine_args(s), s.stream);
             }
             MZB_CHECK(cudaEventRecord(s.ev1, s.stream));
             const int old = G.iphi;

@@ -111,7 +111,7 @@ struct GridState {
     int nu1 = 3, nu2 = 2;
     double batch_cost = 1.0;  // batched-solve time per grid point relative to other sizes (mzb_batch_autotune)
     int lev_plan = -1;        // the plan the current levels were built for
-    void* halo = nullptr;      // work area of the resident CG kernel (ensure_halo)
+    void* halo = nullptr;      // work area of the resident kernels (ensure_halo)
     double* bj_inv = nullptr;  // block-Jacobi block inverse (1000 x 1000) on BLOCKJACOBI grids
     // Poisson-Boltzmann (solver_initialize_grid_pois_boltz, grid_general.c:84-100)
     bool pb = false;
@@ -345,7 +345,7 @@ void set_pb_operator(EngineArgs& a, const PbGrid& g) {
     a.cex = g.cex; a.cey = g.cey; a.cez = g.cez; a.cdg = g.cdg;
 }
 
-// The resident CG kernel's work area, allocated at the first solve that can use it.
+// The resident kernels' work area, allocated at the first solve that can use it.
 void ensure_halo(GridState& G) {
     if (G.halo) return;
     const size_t bytes = resident_halo_bytes(G.n);
@@ -354,7 +354,7 @@ void ensure_halo(GridState& G) {
 
 EngineArgs engine_base(System& s) {
     GridState& G = s.G;
-    if (G.type == G_LCG || G.type == G_MAZE_LCG) ensure_halo(G);
+    ensure_halo(G);
     EngineArgs a{};
     a.n = G.n;
     a.tol = G.tol;
@@ -371,11 +371,11 @@ EngineArgs engine_base(System& s) {
     return a;
 }
 
-// Launch the solver for `a`: the resident kernel where its size and program allow, then the
+// Launch the solver for `a`: the resident kernels where size and program allow, then the
 // TMA-staged CG, then the general engine (MZB_ENGINE=generic: always that).
 void launch_solver(const EngineArgs& a, cudaStream_t stream) {
     static const bool generic_only = getenv("MZB_ENGINE") && strcmp(getenv("MZB_ENGINE"), "generic") == 0;
-    if (!generic_only && (resident_cg_launch(a, stream) || cg_fast_launch(a, stream))) return;
+    if (!generic_only && (resident_cg_launch(a, stream) || resident_mg_launch(a, stream) || cg_fast_launch(a, stream))) return;
     engine_launch(a, stream);
 }
 

@@ -62,6 +62,7 @@ struct ResArgs {
     EngineArgs e;
     int Pi, Pj, cap;   // patches along i and j; elements of one halo strip
     int pairs;         // the most pairs any thread has
+    int cPi, cPj, cpairs, coarse_at;  // the coarse grid's patches and its plane in shared memory (multigrid)
     int smem_doubles;  // dynamic shared memory
     int x_tmem;        // x in tensor memory (else in the grid array it ends in)
     u64 step0;         // halo step numbers of this launch start above this
@@ -90,14 +91,14 @@ struct Shared {
     double res[2];       // a grid-wide sum and its mark count or maximum
     u64 lo[2], hi[2];    // the fixed-point words' values after their last use
     int flag[2];         // [0] a wait ran out, [1] outcome of the last fast_sum
-    int nb[4];           // CTAs of the patches at i - 1, i + 1, j - 1, j + 1
+    int nb[2][4];        // CTAs of the patches at i - 1, i + 1, j - 1, j + 1; [1]: the coarse grid's
     uint32_t tmem;
+    unsigned bulk[kWarps];  // multigrid: bulk_units of the fine grid
 };
-constexpr int kStateDoubles = 32;
+constexpr int kStateDoubles = 48;
 static_assert(sizeof(Shared) <= kStateDoubles * sizeof(double), "state area");
 extern __shared__ __align__(128) double smem[];
 __device__ __forceinline__ Shared& shared_state() { return *reinterpret_cast<Shared*>(smem); }
-__device__ __forceinline__ double* plane() { return smem + kStateDoubles; }
 
 // One CTA's patch of rows, i in [i0, i0 + bi), j in [j0, j0 + bj), whole rows of n points,
 // worked as pairs (k, k + 1). A thread owns one column of pairs (lj, kk) and `cnt` consecutive
@@ -110,9 +111,11 @@ struct Patch {
     int li0, cnt, lj, kk;             // this thread's pairs (cnt = 0: none)
     int o0;                           // its first pair's place in a plane
     int g0, n2;                       // and in the grid; n^2
+    int coarse;                       // 1: a patch of the coarse grid (Shared::nb)
 };
-__device__ __forceinline__ Patch make_patch(int n, int Pi, int Pj) {
+__device__ __forceinline__ Patch make_patch(int n, int Pi, int Pj, int coarse) {
     Patch p;
+    p.coarse = coarse;
     p.n = n;
     p.h = n / 2;
     p.n2 = n * n;
@@ -131,7 +134,7 @@ __device__ __forceinline__ Patch make_patch(int n, int Pi, int Pj) {
     p.bj = (b + 1) * n / Pj - p.j0;
     p.pitch = (p.bj + 2) * n;
     if (threadIdx.x == 0) {
-        int* nb = shared_state().nb;
+        int* nb = shared_state().nb[coarse];
         nb[0] = (a == 0 ? Pi - 1 : a - 1) * Pj + b;
         nb[1] = (a + 1 == Pi ? 0 : a + 1) * Pj + b;
         nb[2] = a * Pj + (b == 0 ? Pj - 1 : b - 1);
@@ -349,8 +352,9 @@ __device__ __forceinline__ bool fixed_point_ok(double prev) {
 // ------------------------------------------------------------------------------------
 // Halo exchange of one value per point of the patch's edge rows.
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ ulonglong2* strip(const ResArgs& a, int cta, u64 step, int side) {
-    return a.strips + ((size_t)(cta * 2 + (int)(step & 1)) * 4 + side) * a.cap;
+// First element of a CTA's strip `side` for a step (the buffers hold fewer than 2^31 elements).
+__device__ __forceinline__ int strip(const ResArgs& a, int cta, u64 step, int side) {
+    return ((cta * 2 + (int)(step & 1)) * 4 + side) * a.cap;
 }
 // Publish unit m's pair if it lies in an edge row: strips 0, 1 hold rows li = 0 and bi - 1
 // (by lj), 2, 3 hold lj = 0 and bj - 1 (by li).
@@ -358,7 +362,7 @@ __device__ __forceinline__ void publish(const ResArgs& a, const Patch& p, int m,
     const int li = p.li0 + m, k = 2 * p.kk;
     const bool e0 = li == 0, e1 = li == p.bi - 1, e2 = p.lj == 0, e3 = p.lj == p.bj - 1;
     if (!(e0 | e1 | e2 | e3)) return;
-    ulonglong2* mine = strip(a, blockIdx.x, step, 0) + k;
+    ulonglong2* mine = a.strips + strip(a, blockIdx.x, step, 0) + k;
     auto put = [&](int side, int row) {
         ulonglong2* d = mine + side * a.cap + row * p.n;
         st_pair(d, v.x, step);
@@ -372,11 +376,11 @@ __device__ __forceinline__ void publish(const ResArgs& a, const Patch& p, int m,
 // Halo row x of the patch (0 .. 2 bi + 2 bj): where it comes from and its place in a shared
 // plane. Rows: li = -1, li = bi (by lj), lj = -1, lj = bj (by li).
 __device__ __forceinline__ int halo_rows(const Patch& p) { return 2 * (p.bi + p.bj); }
-__device__ __forceinline__ const ulonglong2* halo_source(const ResArgs& a, const Patch& p, int x, u64 step) {
+__device__ __forceinline__ int halo_source(const ResArgs& a, const Patch& p, int x, u64 step) {
     const bool along_j = x < 2 * p.bj;
     const int len = along_j ? p.bj : p.bi, y = along_j ? x : x - 2 * p.bj;
     const bool hi = y >= len;
-    const int cta = shared_state().nb[(along_j ? 0 : 2) + (hi ? 1 : 0)];
+    const int cta = shared_state().nb[p.coarse][(along_j ? 0 : 2) + (hi ? 1 : 0)];
     const int side = (along_j ? 0 : 2) + (hi ? 0 : 1);
     return strip(a, cta, step, side) + (hi ? y - len : y) * p.n;
 }
@@ -410,6 +414,33 @@ __device__ __forceinline__ bool receive(const ResArgs& a, const ulonglong2* cons
             all = all && xs[q] == step && ys[q] == step;
             v[q] = make_double2(__longlong_as_double(x[q]), __longlong_as_double(y[q]));
         }
+        if (all) return true;
+        if ((++polls & 255u) == 0u) {
+            const u64 now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (ld_acquire_u32(&a.head->bar.err) != 0u || now - t0 > kBarrierTimeoutNs) {
+                atomicOr(&a.head->bar.err, 1u);
+                return false;
+            }
+        }
+    }
+}
+
+// Wait for NB single values of step `step` at strips + src[q] (negative: none).
+template <int NB>
+__device__ __forceinline__ bool receive_values(const ResArgs& a, const int (&src)[NB], u64 step, u64 (&x)[NB]) {
+    unsigned polls = 0;
+    u64 t0 = 0;
+    for (;;) {
+        u64 xs[NB];
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            xs[q] = step;
+            if (src[q] >= 0) ld_pair(a.strips + src[q], x[q], xs[q]);
+        }
+        bool all = true;
+#pragma unroll
+        for (int q = 0; q < NB; q++) all = all && xs[q] == step;
         if (all) return true;
         if ((++polls & 255u) == 0u) {
             const u64 now = global_ns();
@@ -577,10 +608,9 @@ __device__ __forceinline__ double rz_term(double r) {
 // (library/src/plcg.c:28-238, multigrid.c:13-96, multigrid_pb.c:16-97).
 // ------------------------------------------------------------------------------------
 template <bool PB, int KIND, bool COARSE, int HL>
-__device__ int iterate(const ResArgs& a, Ctl& c, const Patch& p, int units, uint32_t tr, uint32_t tap, uint32_t tx, double* xg,
+__device__ __forceinline__ int iterate(const ResArgs& a, Ctl& c, const Patch& p, int units, double* P, uint32_t tr, uint32_t tap, uint32_t tx, double* xg,
                        const Coef& cf, double rv, double r0, double tol, long limit, bool& ok) {
     Shared& sh = shared_state();
-    double* P = plane();
     double* hs = P + plane_rows(p.n, p.bi, p.bj, units) * p.pitch;
     const double stop = COARSE ? tol * r0 : tol;
     // halo rows of r: warp v >= 1 takes rows v - 1, v + 14, ... and its lanes the row's pairs;
@@ -598,7 +628,7 @@ __device__ int iterate(const ResArgs& a, Ctl& c, const Patch& p, int units, uint
 #pragma unroll
             for (int q = 0; q < NR; q++) {
                 const int row = y + q * (kWarps - 1);
-                const ulonglong2* at = row < nh ? halo_source(a, p, row, c.step) + 2 * lane : nullptr;
+                const ulonglong2* at = a.strips + (row < nh ? halo_source(a, p, row, c.step) : 0) + 2 * lane;
 #pragma unroll
                 for (int t = 0; t < HL; t++)
                     src[q * HL + t] = row < nh && lane + 32 * t < p.h ? at + 64 * t : nullptr;
@@ -890,6 +920,16 @@ __device__ __noinline__ double2 start_residual(const EngineArgs& e, int i, int j
     return make_double2(ax + -1.0 * b, x0);
 }
 
+// Right-hand side of the multigrid programs at one point: c q, for MaZe A (2 phi - phi_prev) + c q
+// (grid_multigrid.c:151-160, verlet.c:108-110).
+template <bool PB>
+__device__ __noinline__ double mg_rhs(const EngineArgs& e, int i, int j, int k) {
+    const Coef cf{e.ex, e.ey, e.ez, e.dg, 0.0, 0.0};
+    const Nb o = nb_of(e.n, i, j, k);
+    if (e.prog == PROG_MG_UPDATE) return e.q[o.c] * e.c;
+    return apply_at<PB>(o, cf, [&](long q) { return 2 * e.phi_old[q] - e.phi_prev[q]; }) + e.c * e.q[o.c];
+}
+
 // conj_grad and its callers. HL: pairs of a row per lane (1 up to n = 64, 2 up to 128).
 template <bool PB, int KIND, int HL>
 __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_constant__ ResArgs a) {
@@ -903,7 +943,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_c
         sh.flag[0] = sh.flag[1] = 0;
         sh.lo[0] = sh.lo[1] = sh.hi[0] = sh.hi[1] = 0;
     }
-    const Patch p = make_patch(n, a.Pi, a.Pj);
+    const Patch p = make_patch(n, a.Pi, a.Pj, 0);
     Ctl c;
     c.step = a.step0;
     const uint32_t tm = tm_alloc(&sh.tmem);
@@ -947,7 +987,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_c
     bool ok = start.ok;
     int result = -1;
     if (ok)
-        result = iterate<PB, KIND, false, HL>(a, c, p, units, tr, tap, tx, xg, cf, KIND == PC_IMPLICIT ? -acc : acc, 0.0, e.tol,
+        result = iterate<PB, KIND, false, HL>(a, c, p, units, smem + kStateDoubles, tr, tap, tx, xg, cf, KIND == PC_IMPLICIT ? -acc : acc, 0.0, e.tol,
                                           (long)n * n, ok);
     if (ok) {
 #pragma unroll 1
@@ -982,11 +1022,416 @@ __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_c
 }
 
 // ------------------------------------------------------------------------------------
+// The reference's two-level multigrid (library/src/multigrid.c:99-168, multigrid_pb.c:270-328)
+// on the same patches, for n a multiple of 4: x in the shared plane, the right-hand side in
+// tensor memory, red-black half-sweeps that exchange the edge rows' new values as iterate()
+// exchanges r's, and the coarse grid (n/2) solved by iterate() on patches of its own. Only
+// the residual before the restriction and the coarse correction pass through global memory,
+// with a grid barrier each.
+//
+// Each function below makes its patch anew: kept in registers across the coarse solve the
+// two patches spilled into it.
+// ------------------------------------------------------------------------------------
+template <bool PB>
+__device__ __forceinline__ Coef fine_coef(const ResArgs& a) {
+    const EngineArgs& e = a.e;
+    return {e.ex, e.ey, e.ez, e.dg, PB ? e.ex[0] : 0.0, PB ? e.dg[0] : 0.0};
+}
+
+// One pair's point of colour (i + j + k) % 2 = colour, e its k parity (multigrid.c:636-729:
+// neighbours i-1, i+1, j-1, j+1, k-1, k+1; multigrid_pb.c:544-640: i+1, i-1, j+1, j-1, k+1, k-1).
+template <bool PB>
+__device__ __forceinline__ double relax(const Patch& p, const double* P, int m, int e, double rhs, const Coef& cf, bool bulk) {
+    const int o = p.o0 + m * p.pitch + e, n = p.n;
+    const double im = P[o - p.pitch], ip = P[o + p.pitch], jm = P[o - n], jp = P[o + n];
+    const double km = P[e == 0 && p.kk == 0 ? o + n - 1 : o - 1], kp = P[e == 1 && p.kk == p.h - 1 ? o + 1 - n : o + 1];
+    if (!PB) {
+        double s = im + ip;
+        s = s + jm;
+        s = s + jp;
+        s = s + km;
+        s = s + kp;
+        return (rhs - s) * (-1.0 / 6.0);
+    }
+    double exc = cf.eb, exm = cf.eb, eyc = cf.eb, eym = cf.eb, ezc = cf.eb, ezm = cf.eb, d = cf.db;
+    if (!bulk) {
+        const int q = m < p.cnt ? m : p.cnt > 0 ? p.cnt - 1 : 0, g = p.g0 + q * p.n2 + e;
+        exc = cf.ex[g];
+        eyc = cf.ey[g];
+        ezc = cf.ez[g];
+        d = cf.dg[g];
+        exm = cf.ex[g + (p.i0 + p.li0 + q == 0 ? (n - 1) * p.n2 : -p.n2)];
+        eym = cf.ey[g + (p.j0 + p.lj == 0 ? (n - 1) * n : -n)];
+        ezm = cf.ez[g + (e == 0 && p.kk == 0 ? n - 1 : -1)];
+    }
+    if (d < 1e-14) d = 1e-14;
+    double s = exc * ip + exm * im;
+    s = s + eyc * jp;
+    s = s + eym * jm;
+    s = s + ezc * kp;
+    s = s + ezm * km;
+    s = s - rhs;
+    return s / d;
+}
+
+// `sweeps` red-black iterations on the plane, its halo current before and after.
+template <bool PB, int HL>
+__device__ __noinline__ bool smooth(const ResArgs& a, Ctl& ctl, uint32_t trhs, int sweeps) {
+    Shared& sh = shared_state();
+    const Patch p = make_patch(a.e.n, a.Pi, a.Pj, 0);
+    const Coef cf = fine_coef<PB>(a);
+    double* P = smem + kStateDoubles;
+    const int units = a.pairs, wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nh = halo_rows(p);
+    const unsigned bulk = PB ? sh.bulk[wid] : 0u;
+    const bool side = p.lj == 0 || p.lj == p.bj - 1;
+    u64 step = ctl.step;
+#pragma unroll 1
+    for (int half = 0; half < 2 * sweeps; half++) {
+        const int colour = half & 1;
+        step++;
+        const int mine = strip(a, blockIdx.x, step, 0);
+#pragma unroll 1
+        for (int m0 = 0; m0 < units; m0 += 2) {
+            Cell t[2];
+            double v[2];
+            int e[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) tm_load(t[q], trhs + 4 * min(m0 + q, units - 1));
+            tm_loaded(t);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int m = min(m0 + q, units - 1);
+                e[q] = (p.i0 + p.li0 + m + p.j0 + p.lj + colour) & 1;
+                const double2 b = pair_of(t[q]);
+                v[q] = relax<PB>(p, P, m, e[q], e[q] ? b.y : b.x, cf, (bulk >> m) & 1u);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int m = m0 + q, li = p.li0 + m;
+                if (m >= p.cnt) continue;
+                P[p.o0 + m * p.pitch + e[q]] = v[q];
+                if (!side && li != 0 && li != p.bi - 1) continue;
+                ulonglong2* d = a.strips + mine + 2 * p.kk + e[q];
+                if (li == 0) st_pair(d + p.lj * p.n, v[q], step);
+                if (li == p.bi - 1) st_pair(d + a.cap + p.lj * p.n, v[q], step);
+                if (p.lj == 0) st_pair(d + 2 * a.cap + li * p.n, v[q], step);
+                if (p.lj == p.bj - 1) st_pair(d + 3 * a.cap + li * p.n, v[q], step);
+            }
+            __syncwarp();
+        }
+        // the neighbours' edge rows, this colour's points; nobody reads this colour meanwhile
+        constexpr int NR = 4 / HL;
+#pragma unroll 1
+        for (int y0 = wid; y0 < nh; y0 += NR * kWarps) {
+            int src[4], dst[4];
+            u64 x[4];
+#pragma unroll
+            for (int q = 0; q < NR; q++) {
+                const int row = y0 + q * kWarps;
+                const bool any = row < nh;
+                const int at = any ? halo_source(a, p, row, step) : 0, to = any ? halo_at(p, row) : 0;
+                const int rows = any ? to / p.n : 0, li = rows / (p.bj + 2) - 1, lj = rows - (li + 1) * (p.bj + 2) - 1;
+                const int e = (p.i0 + li + p.j0 + lj + colour) & 1;
+#pragma unroll
+                for (int t = 0; t < HL; t++) {
+                    const int k = 2 * (lane + 32 * t) + e;
+                    const bool on = any && lane + 32 * t < p.h;
+                    src[q * HL + t] = on ? at + k : -1;
+                    dst[q * HL + t] = to + k;
+                }
+            }
+            if (!receive_values<4>(a, src, step, x)) sh.flag[0] = 1;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (src[q] >= 0) P[dst[q]] = __longlong_as_double(x[q]);
+        }
+        __syncthreads();
+        if (sh.flag[0]) return false;
+    }
+    ctl.step = step;
+    return true;
+}
+
+// rf = -(A x) + rhs into the grid (multigrid.c:113-116), or max |A x - rhs| (the check after
+// each V-cycle, grid_multigrid.c:188-199).
+template <bool PB>
+__device__ __noinline__ double residual(const ResArgs& a, uint32_t trhs, bool store) {
+    const Patch p = make_patch(a.e.n, a.Pi, a.Pj, 0);
+    const Coef cf = fine_coef<PB>(a);
+    const double* P = smem + kStateDoubles;
+    const unsigned bulk = PB ? shared_state().bulk[threadIdx.x >> 5] : 0u;
+    double top = 0.0;
+    double2 im = ld2(P + p.o0 - p.pitch), pc = ld2(P + p.o0);
+#pragma unroll 1
+    for (int m = 0; m < a.pairs; m++) {
+        Cell t[1];
+        tm_load(t[0], trhs + 4 * m);
+        const int o = p.o0 + m * p.pitch;
+        const double2 ip = ld2(P + o + p.pitch);
+        const Around s = around(p, P, o, pc);
+        const double2 v = PB ? apply_pb(s, im, pc, ip, ((bulk >> m) & 1u) ? bulk_faces(cf) : load_faces(p, cf, m))
+                             : apply_lap(s, im, pc, ip);
+        __syncwarp();
+        tm_loaded(t);
+        const double2 b = pair_of(t[0]);
+        if (m < p.cnt) {
+            if (store) st2(a.e.rf + p.g0 + m * p.n2, make_double2(-v.x + 1.0 * b.x, -v.y + 1.0 * b.y));
+            else top = fmax(top, fmax(fabs(v.x + -1.0 * b.x), fabs(v.y + -1.0 * b.y)));
+        }
+        __syncwarp();
+        im = pc;
+        pc = ip;
+    }
+    return top;
+}
+
+// 27-point full weighting of rf at coarse (I, J, K) (multigrid.c:523-594).
+__device__ __noinline__ double restrict_at(const double* in, int n, int I, int J, int K) {
+    const int i = 2 * I, j = 2 * J, k = 2 * K;
+    const int i0 = i * n * n, i1 = (i + 1 == n ? 0 : i + 1) * n * n, i2 = (i == 0 ? n - 1 : i - 1) * n * n;
+    const int j0 = j * n, j1 = (j + 1 == n ? 0 : j + 1) * n, j2 = (j == 0 ? n - 1 : j - 1) * n;
+    const int k1 = (k + 1 == n ? 0 : k + 1), k2 = (k == 0 ? n - 1 : k - 1);
+    auto at = [&](int x) { return __ldcg(in + x); };
+    double f = at(i2 + j0 + k) + at(i1 + j0 + k);
+    f = f + at(i0 + j2 + k);
+    f = f + at(i0 + j1 + k);
+    f = f + at(i0 + j0 + k2);
+    f = f + at(i0 + j0 + k1);
+    double e = at(i1 + j0 + k2) + at(i1 + j0 + k1);
+    e = e + at(i2 + j0 + k2);
+    e = e + at(i2 + j0 + k1);
+    e = e + at(i1 + j2 + k);
+    e = e + at(i1 + j1 + k);
+    e = e + at(i2 + j2 + k);
+    e = e + at(i2 + j1 + k);
+    e = e + at(i0 + j2 + k2);
+    e = e + at(i0 + j2 + k1);
+    e = e + at(i0 + j1 + k2);
+    e = e + at(i0 + j1 + k1);
+    double c = at(i1 + j1 + k2) + at(i1 + j1 + k1);
+    c = c + at(i1 + j2 + k2);
+    c = c + at(i1 + j2 + k1);
+    c = c + at(i2 + j1 + k2);
+    c = c + at(i2 + j1 + k1);
+    c = c + at(i2 + j2 + k2);
+    c = c + at(i2 + j2 + k1);
+    double v = 8.0 * at(i0 + j0 + k) + 4.0 * f;
+    v = v + 2.0 * e;
+    v = v + c;
+    return v * (1.0 / 64.0);
+}
+
+// The coarse correction: A_c e = restriction of rf by CG from zero (50 iterations, relative
+// 1e-5; implicit Jacobi for the Laplacian, none for PB), e into the coarse grid array.
+template <bool PB>
+__device__ __noinline__ bool coarse_solve(const ResArgs& a, Ctl& ctl, uint32_t tm) {
+    constexpr int KIND = PB ? PC_NONE : PC_IMPLICIT;
+    const EngineArgs& e = a.e;
+    Ctl c = ctl;
+    const int nc = e.n / 2, units = a.cpairs;
+    const Patch p = make_patch(nc, a.cPi, a.cPj, 1);
+    const uint32_t tap = tm + 4 * units, tx = tap + 4 * units;
+    const Coef cf{e.cex, e.cey, e.cez, e.cdg, PB ? e.cex[0] : 0.0, PB ? e.cdg[0] : 0.0};
+    double acc = 0.0, top = 0.0;
+#pragma unroll 1
+    for (int m = 0; m < units; m++) {
+        double2 v = make_double2(0.0, 0.0);
+        if (m < p.cnt) {
+            const int I = p.i0 + p.li0 + m, J = p.j0 + p.lj, K = 2 * p.kk;
+            v.x = -1.0 * restrict_at(e.rf, e.n, I, J, K);  // r = A 0 - b
+            v.y = -1.0 * restrict_at(e.rf, e.n, I, J, K + 1);
+            acc += KIND == PC_IMPLICIT ? v.x * (v.x * (1.0 / 6.0)) : v.x * v.x;
+            acc += KIND == PC_IMPLICIT ? v.y * (v.y * (1.0 / 6.0)) : v.y * v.y;
+            top = fmax(top, fmax(fabs(v.x), fabs(v.y)));
+        }
+        __syncwarp();
+        tm_store(tm + 4 * m, v);
+        tm_store(tx + 4 * m, make_double2(0.0, 0.0));
+    }
+    tm_stored();
+    const Reduced start = slow_reduce(a, c.slow_seq++, acc, top);
+    bool ok = start.ok;
+    if (ok && start.max != 0.0)
+        iterate<PB, KIND, true, 1>(a, c, p, units, smem + a.coarse_at, tm, tap, tx, nullptr, cf,
+                                   KIND == PC_IMPLICIT ? -start.sum : start.sum, start.max, 1e-5, 50, ok);
+#pragma unroll 1
+    for (int m = 0; m < units; m++) {
+        Cell t[1];
+        tm_load(t[0], tx + 4 * m);
+        tm_loaded(t);
+        if (m < p.cnt) st2(e.ec + p.g0 + m * p.n2, pair_of(t[0]));
+        __syncwarp();
+    }
+    ctl = c;
+    return ok;
+}
+
+// x += P e on the plane, halo rows included (multigrid.c:393-463: trilinear, weights (1, 0) on
+// even fine indices and (1/2, 1/2) on odd ones).
+__device__ __noinline__ void prolong(const ResArgs& a) {
+    const Patch p = make_patch(a.e.n, a.Pi, a.Pj, 0);
+    double* P = smem + kStateDoubles;
+    const int n = p.n, nc = n / 2, lane = threadIdx.x & 31, nh = halo_rows(p), rows = p.bi * p.bj;
+#pragma unroll 1
+    for (int y = threadIdx.x >> 5; y < rows + nh; y += kWarps) {
+        int li, lj;
+        if (y < rows) {
+            li = y / p.bj;
+            lj = y - li * p.bj;
+        } else {
+            const int r = halo_at(p, y - rows) / n;
+            li = r / (p.bj + 2) - 1;
+            lj = r - (li + 1) * (p.bj + 2) - 1;
+        }
+        int i = p.i0 + li, j = p.j0 + lj;
+        i = i < 0 ? n - 1 : i == n ? 0 : i;
+        j = j < 0 ? n - 1 : j == n ? 0 : j;
+        const int i0 = i >> 1, i1 = i0 + 1 == nc ? 0 : i0 + 1, j0 = j >> 1, j1 = j0 + 1 == nc ? 0 : j0 + 1;
+        const double wi = (i & 1) ? 0.5 : 1.0, wj = (j & 1) ? 0.5 : 1.0;
+        const double* c00 = a.e.ec + (i0 * nc + j0) * nc;
+        const double* c10 = a.e.ec + (i1 * nc + j0) * nc;
+        const double* c01 = a.e.ec + (i0 * nc + j1) * nc;
+        const double* c11 = a.e.ec + (i1 * nc + j1) * nc;
+        double* row = P + ((li + 1) * (p.bj + 2) + lj + 1) * n;
+#pragma unroll 1
+        for (int kk = lane; kk < p.h; kk += 32) {
+            const int k1 = kk + 1 == nc ? 0 : kk + 1;
+            const bool oi = i & 1, oj = j & 1;
+            // the eight weights of prolong_at; those that are zero are left out
+            double e0 = __ldcg(c00 + kk) * wi * wj, o0 = e0 * 0.5, o1 = __ldcg(c00 + k1) * wi * wj * 0.5;
+            double t10[2] = {0.0, 0.0}, t01[2] = {0.0, 0.0}, t11[2] = {0.0, 0.0};
+            if (oi) {
+                t10[0] = __ldcg(c10 + kk) * 0.5 * wj;
+                t10[1] = __ldcg(c10 + k1) * 0.5 * wj * 0.5;
+            }
+            if (oj) {
+                t01[0] = __ldcg(c01 + kk) * wi * 0.5;
+                t01[1] = __ldcg(c01 + k1) * wi * 0.5 * 0.5;
+            }
+            if (oi && oj) {
+                t11[0] = __ldcg(c11 + kk) * 0.5 * 0.5;
+                t11[1] = __ldcg(c11 + k1) * 0.5 * 0.5 * 0.5;
+            }
+            double ev = e0 + t10[0];
+            ev = ev + t01[0];
+            ev = ev + t11[0];
+            double od = o0 + t10[0] * 0.5;
+            od = od + t01[0] * 0.5;
+            od = od + t11[0] * 0.5;
+            od = od + o1;
+            od = od + t10[1];
+            od = od + t01[1];
+            od = od + t11[1];
+            double2 x = ld2(row + 2 * kk);
+            x.x = x.x + 1.0 * ev;
+            x.y = x.y + 1.0 * od;
+            st2(row + 2 * kk, x);
+        }
+    }
+    __syncthreads();
+}
+
+// PROG_MG_UPDATE and PROG_MAZE_MG (grid_multigrid.c:110-212, verlet.c:86-149, 212-271):
+// V-cycles until |A x - b|_inf <= tol, at most 1000.
+template <bool PB, int HL>
+__global__ void __launch_bounds__(kThreads, 1) resident_mg_kernel(const __grid_constant__ ResArgs a) {
+    Shared& sh = shared_state();
+    const EngineArgs& e = a.e;
+    const int n = e.n, units = a.pairs;
+    const bool maze = e.prog == PROG_MAZE_MG;
+    for (int x = threadIdx.x; x < a.smem_doubles; x += kThreads) smem[x] = 0.0;
+    __syncthreads();
+    Ctl c;
+    c.step = a.step0;
+    uint32_t trhs;
+    {
+        const Patch p = make_patch(n, a.Pi, a.Pj, 0);
+        trhs = tm_own(tm_alloc(&sh.tmem));
+        // the start (the MaZe unknown y or the extrapolated field) on the patch and its halo
+        double* P = smem + kStateDoubles;
+        const int lane = threadIdx.x & 31, nh = halo_rows(p), rows = p.bi * p.bj;
+#pragma unroll 1
+        for (int y = threadIdx.x >> 5; y < rows + nh; y += kWarps) {
+            int r = y < rows ? (y / p.bj + 1) * (p.bj + 2) + y % p.bj + 1 : halo_at(p, y - rows) / n;
+            const int li = r / (p.bj + 2) - 1, lj = r - (li + 1) * (p.bj + 2) - 1;
+            int i = p.i0 + li, j = p.j0 + lj;
+            i = i < 0 ? n - 1 : i == n ? 0 : i;
+            j = j < 0 ? n - 1 : j == n ? 0 : j;
+            const int g = (i * n + j) * n;
+            for (int k = lane; k < n; k += 32)
+                P[r * n + k] = maze ? e.y[g + k] : 2 * e.phi_old[g + k] - e.phi_prev[g + k];
+        }
+        const Coef cf = fine_coef<PB>(a);
+        const unsigned bulk = PB ? bulk_units(p, cf, units) : 0u;
+        if (lane == 0) sh.bulk[threadIdx.x >> 5] = bulk;
+#pragma unroll 1
+        for (int m = 0; m < units; m++) {
+            double2 b = make_double2(0.0, 0.0);
+            if (m < p.cnt) {
+                const int i = p.i0 + p.li0 + m, j = p.j0 + p.lj, k = 2 * p.kk;
+                b.x = mg_rhs<PB>(e, i, j, k);
+                b.y = mg_rhs<PB>(e, i, j, k + 1);
+            }
+            __syncwarp();
+            tm_store(trhs + 4 * m, b);
+        }
+        tm_stored();
+        __syncthreads();
+    }
+    const uint32_t tcoarse = trhs + 4 * units;
+    bool ok = true;
+    int result = -1;
+    for (int it = 1; it <= 1000 && ok; it++) {
+        const int sweeps = PB ? 4 : 3;
+        ok = smooth<PB, HL>(a, c, trhs, sweeps);
+        if (!ok) break;
+        residual<PB>(a, trhs, true);
+        ok = grid_sync(&a.head->bar);
+        if (!ok) break;
+        ok = coarse_solve<PB>(a, c, tcoarse);
+        if (!ok) break;
+        ok = grid_sync(&a.head->bar);
+        if (!ok) break;
+        prolong(a);
+        ok = smooth<PB, HL>(a, c, trhs, sweeps);
+        if (!ok) break;
+        const Reduced d = slow_reduce(a, c.slow_seq++, 0.0, residual<PB>(a, trhs, false));
+        ok = d.ok;
+        if (ok && d.max <= e.tol) {
+            result = it;
+            break;
+        }
+    }
+    if (ok) {
+        const Patch p = make_patch(n, a.Pi, a.Pj, 0);
+        const double* P = smem + kStateDoubles;
+#pragma unroll 1
+        for (int m = 0; m < p.cnt; m++) {
+            const int g = p.g0 + m * p.n2;
+            const double2 x = ld2(P + p.o0 + m * p.pitch);
+            if (maze) {  // phi = (2 phi - phi_prev) - y
+                const double2 f = ld2(e.phi_old + g), fp = ld2(e.phi_prev + g);
+                st2(e.y + g, x);
+                st2(e.phi_new + g, make_double2((2 * f.x - fp.x) + -1.0 * x.x, (2 * f.y - fp.y) + -1.0 * x.y));
+            } else {
+                st2(e.phi_new + g, x);
+            }
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        e.result[0] = result;
+        e.result[1] = ok ? 0 : 1;
+    }
+    tm_free(sh.tmem);
+}
+
+// ------------------------------------------------------------------------------------
 // Host: patches, sizes, launch.
 // ------------------------------------------------------------------------------------
 struct Plan {
     int Pi = 0, Pj = 0, bi = 0, bj = 0;
-    int pairs = 0;  // point pairs of the busiest thread
+    int pairs = 0;        // point pairs of the busiest thread
+    size_t plane = 0;     // doubles of the plane of p
     size_t smem = 0;
 };
 constexpr size_t kSmemBudget = 226 * 1024;
@@ -1029,25 +1474,30 @@ Plan find_plan(int n, int sms) {
             const int halo = 2 * (q.bi + q.bj);
             if (q.pairs > kMaxPairs || halo > kMaxHaloSteps * (kWarps - 1)) continue;
             // patches are bi or bi - 1 rows by bj or bj - 1: the largest plane over the four
-            size_t plane = 0;
             for (int bj = n / pj; bj <= q.bj; bj++)
                 for (int bi = n / pi; bi <= q.bi; bi++)
-                    plane = std::max(plane, (size_t)plane_rows(n, bi, bj, q.pairs) * (bj + 2));
-            q.smem = ((plane + halo) * n + kStateDoubles) * sizeof(double);
+                    q.plane = std::max(q.plane, (size_t)plane_rows(n, bi, bj, q.pairs) * (bj + 2) * n);
+            q.smem = (q.plane + (size_t)halo * n + kStateDoubles) * sizeof(double);
             if (q.smem > kSmemBudget) continue;
             if (!best.Pi || q.pairs < best.pairs || (q.pairs == best.pairs && q.bi + q.bj < best.bi + best.bj)) best = q;
         }
     return best;
 }
-const Plan& make_plan(int n, int sms) {  // the last size's plan is kept
-    static thread_local Plan last;
-    static thread_local int last_n = 0, last_sms = 0;
-    if (n != last_n || sms != last_sms) {
-        last = find_plan(n, sms);
-        last_n = n;
-        last_sms = sms;
-    }
-    return last;
+// The last plans are kept (a multigrid launch asks for two).
+Plan make_plan(int n, int sms) {
+    struct Entry {
+        int n = 0, sms = 0;
+        Plan plan;
+    };
+    static thread_local Entry kept[4];
+    static thread_local int next = 0;
+    for (const Entry& e : kept)
+        if (e.n == n && e.sms == sms) return e.plan;
+    Entry& e = kept[next++ & 3];
+    e.n = n;
+    e.sms = sms;
+    e.plan = find_plan(n, sms);
+    return e.plan;
 }
 
 template <int HL>
@@ -1058,6 +1508,28 @@ const void* pick_kernel(bool pb, int kind) {
 }
 
 std::atomic<u64> g_launches{0};
+
+ResArgs common_args(const EngineArgs& e, const Plan& pl) {
+    ResArgs a{};
+    a.e = e;
+    a.Pi = pl.Pi;
+    a.Pj = pl.Pj;
+    a.cap = std::max(pl.bi, pl.bj) * e.n;
+    a.pairs = pl.pairs;
+    a.step0 = ++g_launches << 24;
+    a.head = static_cast<ResHeader*>(e.halo);
+    a.strips = reinterpret_cast<ulonglong2*>(a.head + 1);
+    return a;
+}
+
+void launch(const void* kernel, ResArgs& a, cudaStream_t stream) {
+    const size_t smem = (size_t)a.smem_doubles * sizeof(double);
+    MZB_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    MZB_CHECK(cudaMemsetAsync(a.head, 0, sizeof(ResHeader), stream));
+    void* params[] = {&a};
+    count_launch();
+    MZB_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(a.Pi * a.Pj), dim3(kThreads), params, smem, stream));
+}
 
 }  // namespace
 
@@ -1077,23 +1549,34 @@ bool resident_cg_launch(const EngineArgs& e, cudaStream_t stream) {
     if (kind != PC_IMPLICIT && kind != PC_JACOBI) return false;
     const Plan pl = make_plan(e.n, sm_count());
     if (!pl.Pi) return false;
-    ResArgs a{};
-    a.e = e;
-    a.Pi = pl.Pi;
-    a.Pj = pl.Pj;
-    a.cap = (pl.bi > pl.bj ? pl.bi : pl.bj) * e.n;
-    a.pairs = pl.pairs;
+    ResArgs a = common_args(e, pl);
     a.smem_doubles = (int)(pl.smem / sizeof(double));
     a.x_tmem = pl.pairs <= kMaxPairsX ? 1 : 0;
-    a.step0 = ++g_launches << 24;
-    a.head = static_cast<ResHeader*>(e.halo);
-    a.strips = reinterpret_cast<ulonglong2*>(a.head + 1);
     const void* kf = e.n <= 64 ? pick_kernel<1>(e.pb, kind) : pick_kernel<2>(e.pb, kind);
-    MZB_CHECK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    MZB_CHECK(cudaMemsetAsync(a.head, 0, sizeof(ResHeader), stream));
-    void* params[] = {&a};
-    count_launch();
-    MZB_CHECK(cudaLaunchCooperativeKernel(kf, dim3(pl.Pi * pl.Pj), dim3(kThreads), params, pl.smem, stream));
+    launch(kf, a, stream);
+    return true;
+}
+
+bool resident_mg_launch(const EngineArgs& e, cudaStream_t stream) {
+    if (e.halo == nullptr || (e.prog != PROG_MG_UPDATE && e.prog != PROG_MAZE_MG) || e.n % 4) return false;
+    const Plan pl = make_plan(e.n, sm_count());
+    if (!pl.Pi) return false;
+    const Plan cp = make_plan(e.n / 2, pl.Pi * pl.Pj);  // the fine grid's CTAs, some without a coarse patch
+    if (!cp.Pi || 4 * pl.pairs + 12 * cp.pairs > 128) return false;
+    ResArgs a = common_args(e, pl);
+    a.cPi = cp.Pi;
+    a.cPj = cp.Pj;
+    a.cpairs = cp.pairs;
+    a.coarse_at = kStateDoubles + (int)pl.plane;
+    // the coarse plane and halo rows, and what a CTA without a patch reads for nothing
+    const int coarse = std::max((int)(cp.smem / sizeof(double)) - kStateDoubles, (cp.pairs + 3) * e.n);
+    a.smem_doubles = a.coarse_at + coarse;
+    const int ccap = std::max(cp.bi, cp.bj) * (e.n / 2);
+    if (a.smem_doubles * sizeof(double) > kSmemBudget || ccap > a.cap) return false;
+    const bool one = e.n <= 64;
+    launch(e.pb ? (one ? (const void*)resident_mg_kernel<true, 1> : (const void*)resident_mg_kernel<true, 2>)
+                : (one ? (const void*)resident_mg_kernel<false, 1> : (const void*)resident_mg_kernel<false, 2>),
+           a, stream);
     return true;
 }
 

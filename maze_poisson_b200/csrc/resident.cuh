@@ -15,4 +15,8 @@ size_t resident_halo_bytes(int n);
 // the device does not allow it, or without a work area.
 bool resident_cg_launch(const EngineArgs& a, cudaStream_t stream);
 
+// Launch PROG_MG_UPDATE or PROG_MAZE_MG (either operator) on the resident multigrid kernel;
+// false when the grid is not a multiple of 4, too large, or has no work area.
+bool resident_mg_launch(const EngineArgs& a, cudaStream_t stream);
+
 }  // namespace mzb

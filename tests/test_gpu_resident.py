@@ -11,7 +11,9 @@ meets the solver's tolerance up to the rounding between the recursive and the tr
 import numpy as np
 import pytest
 
+import mdparity
 from maze_poisson_b200.c_api import CAPI
+from maze_poisson_b200.systems import make_melt, make_pb_system, pb_settings
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-6
@@ -86,3 +88,23 @@ def test_cg_out_of_fixed_point_range(lib, oracle_lib, power):
     assert abs(lib.mzb_conj_grad(b * s, x0 * s, y, TOL * s, n, 0) - it) <= 1
     assert rel(y / s, x) < 1e-5
     assert np.isfinite(y).all()
+
+
+@pytest.mark.parametrize("n,ions,method,pb", [(32, 128, "MULTIGRID", False), (64, 250, "MAZE-MULTIGRID", False),
+                                              (68, 250, "MULTIGRID", False), (84, 432, "MAZE-MULTIGRID", False),
+                                              (32, 8, "MAZE-MULTIGRID", True), (68, 8, "MULTIGRID", True)])
+def test_multigrid_sizes(lib, oracle_path, n, ions, method, pb):
+    """The resident multigrid kernel in MD steps: patches of the coarse grid that fill the
+    CTAs and that leave some without, one and two pairs of a row per lane. The V-cycle amplifies
+    the order of the coarse CG's sums, so the bound is five times the oracle's own change under
+    a 1e-15 scaling of the positions, at least 1e-10."""
+    orc = CAPI(oracle_path, extensions=False)
+    kw = dict(method=method, tol=1e-10, integrator="VERLET")
+    if pb:
+        system = make_pb_system(ions, n, 0.5 * n, seed=n)
+        kw.update(pb=pb_settings(system), eps_s=78.4, eps_int=1.0, T=300.0)
+    else:
+        system = make_melt(ions, n, seed=n)
+    floor = mdparity.oracle_floor(orc, system, 2, **kw)
+    bounds = {k: max(1e-10, 5 * floor["fcs_elec"], 5 * floor["fcs_tot"]) for k in ("fcs_elec", "fcs_tot", "vel")}
+    mdparity.run_pair(lib, orc, system, 2, bounds=bounds, **kw)

@@ -234,7 +234,11 @@ __device__ __forceinline__ bool block_total(double& v, bool any) {
     v = warp_sum(v);
     if ((threadIdx.x & 31) == 0) sh.sum[threadIdx.x >> 5] = v;
     const bool r = __syncthreads_or(any);
-    if (threadIdx.x < 32) v = warp_sum(threadIdx.x < kWarps ? sh.sum[threadIdx.x] : 0.0);
+    if (threadIdx.x < kWarps) {
+        v = sh.sum[threadIdx.x];
+#pragma unroll
+        for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync((1u << kWarps) - 1u, v, o);
+    }
     return r;
 }
 
@@ -426,6 +430,14 @@ __device__ __forceinline__ bool receive(const ResArgs& a, const ulonglong2* cons
     }
 }
 
+// k parity of colour's points in halo row x.
+__device__ __forceinline__ int halo_parity(const Patch& p, int x, int colour) {
+    const bool along_j = x < 2 * p.bj;
+    const int len = along_j ? p.bj : p.bi, y = along_j ? x : x - 2 * p.bj;
+    const bool hi = y >= len;
+    const int at = hi ? y - len : y, far = hi ? (along_j ? p.bi : p.bj) : -1;
+    return (p.i0 + p.j0 + at + far + colour) & 1;
+}
 // Wait for NB single values of step `step` at strips + src[q] (negative: none).
 template <int NB>
 __device__ __forceinline__ bool receive_values(const ResArgs& a, const int (&src)[NB], u64 step, u64 (&x)[NB]) {
@@ -1031,6 +1043,13 @@ __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_c
 //
 // Each function below makes its patch anew: kept in registers across the coarse solve the
 // two patches spilled into it.
+//
+// Measured on one B200, us per V-cycle, before (engine.cu) and now: 64^3 609 / 271, 96^3 714 /
+// 318, 128^3 843 / 392, Poisson-Boltzmann 96^3 819 / 399, 128^3 1019 / 631. 230 to 290 us of it are the 50 coarse
+// iterations (4.6 us each at 32^3, 5.5 at 64^3: the latency of two sums and a halo trip), a
+// half-sweep takes 2.1 us at 64^3 and 7 us at 128^3 (issue). Tried: the coarse rows of the
+// correction staged in shared memory (prolong 13 instead of 10 us), the next points' PB
+// coefficients loaded ahead (spills: 59 instead of 47 us for four sweeps at 96^3).
 // ------------------------------------------------------------------------------------
 template <bool PB>
 __device__ __forceinline__ Coef fine_coef(const ResArgs& a) {
@@ -1038,85 +1057,113 @@ __device__ __forceinline__ Coef fine_coef(const ResArgs& a) {
     return {e.ex, e.ey, e.ez, e.dg, PB ? e.ex[0] : 0.0, PB ? e.dg[0] : 0.0};
 }
 
-// One pair's point of colour (i + j + k) % 2 = colour, e its k parity (multigrid.c:636-729:
-// neighbours i-1, i+1, j-1, j+1, k-1, k+1; multigrid_pb.c:544-640: i+1, i-1, j+1, j-1, k+1, k-1).
-template <bool PB>
-__device__ __forceinline__ double relax(const Patch& p, const double* P, int m, int e, double rhs, const Coef& cf, bool bulk) {
-    const int o = p.o0 + m * p.pitch + e, n = p.n;
-    const double im = P[o - p.pitch], ip = P[o + p.pitch], jm = P[o - n], jp = P[o + n];
-    const double km = P[e == 0 && p.kk == 0 ? o + n - 1 : o - 1], kp = P[e == 1 && p.kk == p.h - 1 ? o + 1 - n : o + 1];
-    if (!PB) {
-        double s = im + ip;
-        s = s + jm;
-        s = s + jp;
-        s = s + km;
-        s = s + kp;
-        return (rhs - s) * (-1.0 / 6.0);
-    }
-    double exc = cf.eb, exm = cf.eb, eyc = cf.eb, eym = cf.eb, ezc = cf.eb, ezm = cf.eb, d = cf.db;
+// The Poisson-Boltzmann coefficients around one point.
+struct PointFaces {
+    double exc, exm, eyc, eym, ezc, ezm, d;
+};
+__device__ __forceinline__ PointFaces point_faces(const Patch& p, const Coef& cf, int m, int e, bool bulk) {
+    PointFaces f = {cf.eb, cf.eb, cf.eb, cf.eb, cf.eb, cf.eb, cf.db};
     if (!bulk) {
-        const int q = m < p.cnt ? m : p.cnt > 0 ? p.cnt - 1 : 0, g = p.g0 + q * p.n2 + e;
-        exc = cf.ex[g];
-        eyc = cf.ey[g];
-        ezc = cf.ez[g];
-        d = cf.dg[g];
-        exm = cf.ex[g + (p.i0 + p.li0 + q == 0 ? (n - 1) * p.n2 : -p.n2)];
-        eym = cf.ey[g + (p.j0 + p.lj == 0 ? (n - 1) * n : -n)];
-        ezm = cf.ez[g + (e == 0 && p.kk == 0 ? n - 1 : -1)];
+        const int q = m < p.cnt ? m : p.cnt > 0 ? p.cnt - 1 : 0, g = p.g0 + q * p.n2 + e, n = p.n;
+        f.exc = cf.ex[g];
+        f.eyc = cf.ey[g];
+        f.ezc = cf.ez[g];
+        f.d = cf.dg[g];
+        f.exm = cf.ex[g + (p.i0 + p.li0 + q == 0 ? (n - 1) * p.n2 : -p.n2)];
+        f.eym = cf.ey[g + (p.j0 + p.lj == 0 ? (n - 1) * n : -n)];
+        f.ezm = cf.ez[g + (e == 0 && p.kk == 0 ? n - 1 : -1)];
     }
-    if (d < 1e-14) d = 1e-14;
-    double s = exc * ip + exm * im;
-    s = s + eyc * jp;
-    s = s + eym * jm;
-    s = s + ezc * kp;
-    s = s + ezm * km;
-    s = s - rhs;
-    return s / d;
+    return f;
 }
 
-// `sweeps` red-black iterations on the plane, its halo current before and after.
+// `sweeps` red-black iterations on the plane, its halo current before and after: the points
+// with (i + j + k) even, then odd (multigrid.c:636-729, neighbours i-1, i+1, j-1, j+1, k-1,
+// k+1; multigrid_pb.c:544-640, i+1, i-1, j+1, j-1, k+1, k-1).
+//
+// Of each pair one element belongs to the colour, and it alternates along the column. The
+// other element of row m is the pair's inner k neighbour of unit m and, at the same time, the
+// i neighbour of units m - 1 and m + 1: one load per row serves three, and a unit takes four
+// shared-memory loads instead of seven. Two units' loads and sums run together.
 template <bool PB, int HL>
 __device__ __noinline__ bool smooth(const ResArgs& a, Ctl& ctl, uint32_t trhs, int sweeps) {
     Shared& sh = shared_state();
     const Patch p = make_patch(a.e.n, a.Pi, a.Pj, 0);
     const Coef cf = fine_coef<PB>(a);
     double* P = smem + kStateDoubles;
-    const int units = a.pairs, wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nh = halo_rows(p);
+    const int n = p.n, units = a.pairs, wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nh = halo_rows(p);
     const unsigned bulk = PB ? sh.bulk[wid] : 0u;
     const bool side = p.lj == 0 || p.lj == p.bj - 1;
     u64 step = ctl.step;
 #pragma unroll 1
     for (int half = 0; half < 2 * sweeps; half++) {
-        const int colour = half & 1;
+        const int colour = half & 1, e0 = (p.i0 + p.li0 + p.j0 + p.lj + colour) & 1;
+        // the outer k neighbour's distance from the first element of the pair, by e
+        const int out0 = p.kk == 0 ? n - 1 : -1, out1 = p.kk == p.h - 1 ? 2 - n : 2;
         step++;
-        const int mine = strip(a, blockIdx.x, step, 0);
+        ulonglong2* mine = a.strips + strip(a, blockIdx.x, step, 0) + 2 * p.kk;
+        // the elements that are not this colour's in rows m0 - 1 and m0
+        double wm = P[p.o0 - p.pitch + e0], w0 = P[p.o0 + (e0 ^ 1)];
 #pragma unroll 1
         for (int m0 = 0; m0 < units; m0 += 2) {
+            const bool two = m0 + 1 < units;
+            const int o = p.o0 + m0 * p.pitch, o1 = two ? o + p.pitch : o;
             Cell t[2];
-            double v[2];
-            int e[2];
-#pragma unroll
-            for (int q = 0; q < 2; q++) tm_load(t[q], trhs + 4 * min(m0 + q, units - 1));
+            tm_load(t[0], trhs + 4 * m0);
+            tm_load(t[1], trhs + 4 * (two ? m0 + 1 : m0));
+            // rows m0 + 1 and m0 + 2
+            const double w1 = P[o + p.pitch + e0], w2 = P[o1 + p.pitch + (e0 ^ 1)];
+            const double k0 = P[o + (e0 ? out1 : out0)], k1 = P[o1 + (e0 ? out0 : out1)];
+            const double jm0 = P[o - n + e0], jp0 = P[o + n + e0];
+            const double jm1 = P[o1 - n + (e0 ^ 1)], jp1 = P[o1 + n + (e0 ^ 1)];
             tm_loaded(t);
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int m = min(m0 + q, units - 1);
-                e[q] = (p.i0 + p.li0 + m + p.j0 + p.lj + colour) & 1;
-                const double2 b = pair_of(t[q]);
-                v[q] = relax<PB>(p, P, m, e[q], e[q] ? b.y : b.x, cf, (bulk >> m) & 1u);
+            const double2 b0 = pair_of(t[0]), b1 = pair_of(t[1]);
+            const double r0 = e0 ? b0.y : b0.x, r1 = e0 ? b1.x : b1.y;
+            const double km0 = e0 ? w0 : k0, kp0 = e0 ? k0 : w0, km1 = e0 ? k1 : w1, kp1 = e0 ? w1 : k1;
+            double v0, v1;
+            if (!PB) {
+                double s0 = wm + w1, s1 = w0 + w2;
+                s0 = s0 + jm0;
+                s1 = s1 + jm1;
+                s0 = s0 + jp0;
+                s1 = s1 + jp1;
+                s0 = s0 + km0;
+                s1 = s1 + km1;
+                s0 = s0 + kp0;
+                s1 = s1 + kp1;
+                v0 = (r0 - s0) * (-1.0 / 6.0);
+                v1 = (r1 - s1) * (-1.0 / 6.0);
+            } else {
+                const PointFaces f = point_faces(p, cf, m0, e0, (bulk >> m0) & 1u);
+                const PointFaces g = point_faces(p, cf, m0 + 1, e0 ^ 1, (bulk >> (m0 + 1)) & 1u);
+                double s0 = f.exc * w1 + f.exm * wm, s1 = g.exc * w2 + g.exm * w0;
+                s0 = s0 + f.eyc * jp0;
+                s1 = s1 + g.eyc * jp1;
+                s0 = s0 + f.eym * jm0;
+                s1 = s1 + g.eym * jm1;
+                s0 = s0 + f.ezc * kp0;
+                s1 = s1 + g.ezc * kp1;
+                s0 = s0 + f.ezm * km0;
+                s1 = s1 + g.ezm * km1;
+                s0 = s0 - r0;
+                s1 = s1 - r1;
+                v0 = s0 / (f.d < 1e-14 ? 1e-14 : f.d);
+                v1 = s1 / (g.d < 1e-14 ? 1e-14 : g.d);
             }
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int m = m0 + q, li = p.li0 + m;
-                if (m >= p.cnt) continue;
-                P[p.o0 + m * p.pitch + e[q]] = v[q];
-                if (!side && li != 0 && li != p.bi - 1) continue;
-                ulonglong2* d = a.strips + mine + 2 * p.kk + e[q];
-                if (li == 0) st_pair(d + p.lj * p.n, v[q], step);
-                if (li == p.bi - 1) st_pair(d + a.cap + p.lj * p.n, v[q], step);
-                if (p.lj == 0) st_pair(d + 2 * a.cap + li * p.n, v[q], step);
-                if (p.lj == p.bj - 1) st_pair(d + 3 * a.cap + li * p.n, v[q], step);
-            }
+            wm = w1;
+            w0 = w2;
+            auto put = [&](int m, int e, double v) {
+                if (m >= p.cnt) return;
+                const int li = p.li0 + m;
+                P[p.o0 + m * p.pitch + e] = v;
+                if (!side && li != 0 && li != p.bi - 1) return;
+                ulonglong2* d = mine + e;
+                if (li == 0) st_pair(d + p.lj * n, v, step);
+                if (li == p.bi - 1) st_pair(d + a.cap + p.lj * n, v, step);
+                if (p.lj == 0) st_pair(d + 2 * a.cap + li * n, v, step);
+                if (p.lj == p.bj - 1) st_pair(d + 3 * a.cap + li * n, v, step);
+            };
+            put(m0, e0, v0);
+            if (two) put(m0 + 1, e0 ^ 1, v1);
             __syncwarp();
         }
         // the neighbours' edge rows, this colour's points; nobody reads this colour meanwhile
@@ -1130,8 +1177,7 @@ __device__ __noinline__ bool smooth(const ResArgs& a, Ctl& ctl, uint32_t trhs, i
                 const int row = y0 + q * kWarps;
                 const bool any = row < nh;
                 const int at = any ? halo_source(a, p, row, step) : 0, to = any ? halo_at(p, row) : 0;
-                const int rows = any ? to / p.n : 0, li = rows / (p.bj + 2) - 1, lj = rows - (li + 1) * (p.bj + 2) - 1;
-                const int e = (p.i0 + li + p.j0 + lj + colour) & 1;
+                const int e = halo_parity(p, row, colour);
 #pragma unroll
                 for (int t = 0; t < HL; t++) {
                     const int k = 2 * (lane + 32 * t) + e;
@@ -1185,40 +1231,57 @@ __device__ __noinline__ double residual(const ResArgs& a, uint32_t trhs, bool st
     return top;
 }
 
-// 27-point full weighting of rf at coarse (I, J, K) (multigrid.c:523-594).
-__device__ __noinline__ double restrict_at(const double* in, int n, int I, int J, int K) {
+// 27-point full weighting of rf at coarse (I, J, K) and (I, J, K + 1), K even
+// (multigrid.c:523-594): the nine rows' five values each, all loads before the sums.
+__device__ __noinline__ double2 restrict_pair(const double* in, int n, int I, int J, int K) {
     const int i = 2 * I, j = 2 * J, k = 2 * K;
-    const int i0 = i * n * n, i1 = (i + 1 == n ? 0 : i + 1) * n * n, i2 = (i == 0 ? n - 1 : i - 1) * n * n;
-    const int j0 = j * n, j1 = (j + 1 == n ? 0 : j + 1) * n, j2 = (j == 0 ? n - 1 : j - 1) * n;
-    const int k1 = (k + 1 == n ? 0 : k + 1), k2 = (k == 0 ? n - 1 : k - 1);
-    auto at = [&](int x) { return __ldcg(in + x); };
-    double f = at(i2 + j0 + k) + at(i1 + j0 + k);
-    f = f + at(i0 + j2 + k);
-    f = f + at(i0 + j1 + k);
-    f = f + at(i0 + j0 + k2);
-    f = f + at(i0 + j0 + k1);
-    double e = at(i1 + j0 + k2) + at(i1 + j0 + k1);
-    e = e + at(i2 + j0 + k2);
-    e = e + at(i2 + j0 + k1);
-    e = e + at(i1 + j2 + k);
-    e = e + at(i1 + j1 + k);
-    e = e + at(i2 + j2 + k);
-    e = e + at(i2 + j1 + k);
-    e = e + at(i0 + j2 + k2);
-    e = e + at(i0 + j2 + k1);
-    e = e + at(i0 + j1 + k2);
-    e = e + at(i0 + j1 + k1);
-    double c = at(i1 + j1 + k2) + at(i1 + j1 + k1);
-    c = c + at(i1 + j2 + k2);
-    c = c + at(i1 + j2 + k1);
-    c = c + at(i2 + j1 + k2);
-    c = c + at(i2 + j1 + k1);
-    c = c + at(i2 + j2 + k2);
-    c = c + at(i2 + j2 + k1);
-    double v = 8.0 * at(i0 + j0 + k) + 4.0 * f;
-    v = v + 2.0 * e;
-    v = v + c;
-    return v * (1.0 / 64.0);
+    const int gi[3] = {i * n * n, (i + 1 == n ? 0 : i + 1) * n * n, (i == 0 ? n - 1 : i - 1) * n * n};
+    const int gj[3] = {j * n, (j + 1 == n ? 0 : j + 1) * n, (j == 0 ? n - 1 : j - 1) * n};
+    const int km = k == 0 ? n - 1 : k - 1;
+    double v[3][3][5];  // [i, i + 1, i - 1][j, j + 1, j - 1][k - 1 .. k + 3]
+#pragma unroll
+    for (int x = 0; x < 3; x++)
+#pragma unroll
+        for (int y = 0; y < 3; y++) {
+            const double* row = in + gi[x] + gj[y];
+            const double2 lo = __ldcg(reinterpret_cast<const double2*>(row + k));
+            const double2 hi = __ldcg(reinterpret_cast<const double2*>(row + k + 2));
+            v[x][y][0] = __ldcg(row + km);
+            v[x][y][1] = lo.x;
+            v[x][y][2] = lo.y;
+            v[x][y][3] = hi.x;
+            v[x][y][4] = hi.y;
+        }
+    auto weigh = [&](int c) {  // centre at value c
+        double f = v[2][0][c] + v[1][0][c];
+        f = f + v[0][2][c];
+        f = f + v[0][1][c];
+        f = f + v[0][0][c - 1];
+        f = f + v[0][0][c + 1];
+        double e = v[1][0][c - 1] + v[1][0][c + 1];
+        e = e + v[2][0][c - 1];
+        e = e + v[2][0][c + 1];
+        e = e + v[1][2][c];
+        e = e + v[1][1][c];
+        e = e + v[2][2][c];
+        e = e + v[2][1][c];
+        e = e + v[0][2][c - 1];
+        e = e + v[0][2][c + 1];
+        e = e + v[0][1][c - 1];
+        e = e + v[0][1][c + 1];
+        double q = v[1][1][c - 1] + v[1][1][c + 1];
+        q = q + v[1][2][c - 1];
+        q = q + v[1][2][c + 1];
+        q = q + v[2][1][c - 1];
+        q = q + v[2][1][c + 1];
+        q = q + v[2][2][c - 1];
+        q = q + v[2][2][c + 1];
+        double s = 8.0 * v[0][0][c] + 4.0 * f;
+        s = s + 2.0 * e;
+        s = s + q;
+        return s * (1.0 / 64.0);
+    };
+    return make_double2(weigh(1), weigh(3));
 }
 
 // The coarse correction: A_c e = restriction of rf by CG from zero (50 iterations, relative
@@ -1238,8 +1301,8 @@ __device__ __noinline__ bool coarse_solve(const ResArgs& a, Ctl& ctl, uint32_t t
         double2 v = make_double2(0.0, 0.0);
         if (m < p.cnt) {
             const int I = p.i0 + p.li0 + m, J = p.j0 + p.lj, K = 2 * p.kk;
-            v.x = -1.0 * restrict_at(e.rf, e.n, I, J, K);  // r = A 0 - b
-            v.y = -1.0 * restrict_at(e.rf, e.n, I, J, K + 1);
+            const double2 b = restrict_pair(e.rf, e.n, I, J, K);
+            v = make_double2(-1.0 * b.x, -1.0 * b.y);  // r = A 0 - b
             acc += KIND == PC_IMPLICIT ? v.x * (v.x * (1.0 / 6.0)) : v.x * v.x;
             acc += KIND == PC_IMPLICIT ? v.y * (v.y * (1.0 / 6.0)) : v.y * v.y;
             top = fmax(top, fmax(fabs(v.x), fabs(v.y)));

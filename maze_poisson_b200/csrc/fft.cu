@@ -5,7 +5,7 @@
 //   I  : forward along i, multiply by ig2, inverse along i (one read, one write)
 //   J' : inverse along j
 //   K' : c2r along k
-// For n = 64, 128 and 256 each 1-D transform runs in registers (see solve_reg); other
+// For the sizes of reg_solver each 1-D transform runs in registers (see solve_reg); other
 // sizes run each 1-D transform in shared memory as a mixed-radix (4, 2, 3) Stockham FFT.
 // Both use an accurate twiddle table (sincospi). Reference semantics (library/src/grid_fft.c:65-125,
 // fftw_wrap.c:166-189): ig2 = 4 pi / (h^3 n^3) / (k^2 + 1e-10) with continuous
@@ -253,205 +253,246 @@ __global__ void __launch_bounds__(kFftThreads) k_pass_cols(double2* __restrict__
     }
 }
 
-// ---- register-resident transforms for n = 64, 128, 256 ----
+// ---- register-resident transforms for n = N1 N2 (reg_solver below lists the sizes) ----
 //
 // A length-N transform is split N = N1 x N2 (Cooley-Tukey, four-step): N2 threads work it,
 // thread t holding x[n1 N2 + t] for n1 < N1; each forms a length-N1 DFT in registers,
 // multiplies by W_N^(t k1), the partial results are exchanged through shared memory, and
-// each thread forms the length-N2 DFTs of its k1 = t + N2 a, ending with X[k1 + N1 k2].
-// That output set is again {m : m = t mod N2}, the input distribution, so an inverse can
-// start from registers. Small DFTs are radix-2 decimation-in-time with compile-time
-// indices; every twiddle comes from the accurate table W (exp(-2 pi i m / N), sincospi).
-// The passes move each value once each way with whole 128-byte segments per warp, and no
-// integer division is left in the butterflies.
-template <int N> struct Split;
-template <> struct Split<256> { static constexpr int N1 = 16, N2 = 16; };
-template <> struct Split<128> { static constexpr int N1 = 16, N2 = 8; };
-template <> struct Split<64> { static constexpr int N1 = 8, N2 = 8; };
-// exchange buffer of one sequence: N1 rows of N2 + 1 doubles, plus 4 so that consecutive
-// sequences' buffers start 8 banks apart
-template <int N> constexpr int XchLen = Split<N>::N1 * (Split<N>::N2 + 1) + 4;
-
-__host__ __device__ constexpr int ilog2(int v) { return v >= 16 ? 4 : v >= 8 ? 3 : v >= 4 ? 2 : v >= 2 ? 1 : 0; }
-// bit reversal of v in `bits` (<= 4) bits
-__host__ __device__ constexpr int bitrev(int v, int bits) {
-    const int r4 = ((v & 1) << 3) | ((v & 2) << 1) | ((v & 4) >> 1) | ((v & 8) >> 3);
-    return r4 >> (4 - bits);
-}
-
-// In-register DFT of length R on (xr, xi) (natural order in and out); w holds W_N^m and
-// W_R^j = w[j * (N / R)].
-// one radix-2 stage of span M = 2^S over the R registers (compile-time indices)
-template <int R, int N, bool INV, int M>
-__device__ __forceinline__ void dit_stage(double (&xr)[R], double (&xi)[R], const double2* w) {
-    constexpr int H = M / 2;
-#pragma unroll
-    for (int k = 0; k < R; k += M) {
-#pragma unroll
-        for (int j = 0; j < H; j++) {
-            const double br = xr[k + j + H], bi = xi[k + j + H];
-            double tr = br, ti = bi;
-            if (j != 0) {
-                const double2 tw = w[j * (N / M)];
-                const double c = tw.x, sn = INV ? -tw.y : tw.y;
-                tr = fma(br, c, -bi * sn);
-                ti = fma(br, sn, bi * c);
-            }
-            const double ur = xr[k + j], ui = xi[k + j];
-            xr[k + j] = ur + tr;
-            xi[k + j] = ui + ti;
-            xr[k + j + H] = ur - tr;
-            xi[k + j + H] = ui - ti;
-        }
-    }
-}
-
+// each thread forms the length-N2 DFTs of its k1 = t, t + N2, ... < N1, ending with
+// X[k1 + N1 k2]. The inverse after the i pass's multiplication takes the same steps
+// backwards from those registers. The small DFTs (N1, N2 <= 18) are recursive mixed radix 4,
+// 2, 3 with compile-time indices; every twiddle comes from the accurate table W
+// (exp(-2 pi i m / N), sincospi). The passes move each value once each way with whole
+// 128-byte segments per warp, and no integer division is left in the butterflies: the
+// shared-memory Stockham kernels above spent their time there (144^3: 544 us per solve in
+// five passes that move 48 MB each from L2).
 template <int R, int N, bool INV>
 __device__ __forceinline__ void dft_reg(double (&xr)[R], double (&xi)[R], const double2* w) {
-    constexpr int B = ilog2(R);
+    if constexpr (R == 1) {
+    } else if constexpr (R == 2) {
+        const double tr = xr[0] - xr[1], ti = xi[0] - xi[1];
+        xr[0] = xr[0] + xr[1];
+        xi[0] = xi[0] + xi[1];
+        xr[1] = tr;
+        xi[1] = ti;
+    } else if constexpr (R == 3) {
+        const double s3 = 0.86602540378443864676;  // sqrt(3)/2
+        const double tr = xr[1] + xr[2], ti = xi[1] + xi[2];
+        const double ur = fma(-0.5, tr, xr[0]), ui = fma(-0.5, ti, xi[0]);
+        const double dr = xr[1] - xr[2], di = xi[1] - xi[2];
+        // -i s3 (x1 - x2) forward, +i s3 (x1 - x2) inverse
+        const double vr = INV ? -s3 * di : s3 * di, vi = INV ? s3 * dr : -s3 * dr;
+        xr[0] = xr[0] + tr;
+        xi[0] = xi[0] + ti;
+        xr[1] = ur + vr;
+        xi[1] = ui + vi;
+        xr[2] = ur - vr;
+        xi[2] = ui - vi;
+    } else if constexpr (R == 4) {
+        const double ar = xr[0] + xr[2], ai = xi[0] + xi[2], br = xr[0] - xr[2], bi = xi[0] - xi[2];
+        const double cr = xr[1] + xr[3], ci = xi[1] + xi[3], er = xr[1] - xr[3], ei = xi[1] - xi[3];
+        // -i (x1 - x3) forward, +i (x1 - x3) inverse
+        const double dr = INV ? -ei : ei, di = INV ? er : -er;
+        xr[0] = ar + cr;
+        xi[0] = ai + ci;
+        xr[1] = br + dr;
+        xi[1] = bi + di;
+        xr[2] = ar - cr;
+        xi[2] = ai - ci;
+        xr[3] = br - dr;
+        xi[3] = bi - di;
+    } else {  // R = P Q: P length-Q DFTs of the decimated sequences, combined by length-P DFTs
+        constexpr int P = R % 4 == 0 ? 4 : R % 3 == 0 ? 3 : 2, Q = R / P;
+        static_assert(P * Q == R, "lengths are 2^a 3^b");
+        double ar[P][Q], ai[P][Q];
 #pragma unroll
-    for (int q = 0; q < R; q++) {  // bit-reversal permutation, in place
-        const int p = bitrev(q, B);
-        if (q < p) {
-            const double tr = xr[q], ti = xi[q];
-            xr[q] = xr[p];
-            xi[q] = xi[p];
-            xr[p] = tr;
-            xi[p] = ti;
+        for (int p = 0; p < P; p++) {
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                ar[p][q] = xr[q * P + p];
+                ai[p][q] = xi[q * P + p];
+            }
+            dft_reg<Q, N, INV>(ar[p], ai[p], w);
+        }
+#pragma unroll
+        for (int k = 0; k < Q; k++) {
+            double yr[P], yi[P];
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                yr[p] = ar[p][k];
+                yi[p] = ai[p][k];
+                if (p * k != 0) {
+                    const double2 tw = w[p * k * (N / R)];
+                    const double c = tw.x, sn = INV ? -tw.y : tw.y, r = yr[p];
+                    yr[p] = fma(r, c, -yi[p] * sn);
+                    yi[p] = fma(r, sn, yi[p] * c);
+                }
+            }
+            dft_reg<P, N, INV>(yr, yi, w);
+#pragma unroll
+            for (int m = 0; m < P; m++) {
+                xr[k + Q * m] = yr[m];
+                xi[k + Q * m] = yi[m];
+            }
         }
     }
-    dit_stage<R, N, INV, 2>(xr, xi, w);
-    dit_stage<R, N, INV, 4>(xr, xi, w);
-    dit_stage<R, N, INV, 8>(xr, xi, w);
-    if constexpr (R >= 16) dit_stage<R, N, INV, 16>(xr, xi, w);
 }
 
-// The distributed length-N transform of one sequence by its N2 threads (t = this thread's
-// rank): in, xr[n1] = x[n1 N2 + t]; out, xr[a N2 + k2] = X[(t + N2 a) + N1 k2]. (xre, xim)
-// is the sequence's exchange buffer (XchLen<N> doubles each: N1 rows of N2 + 1, the pad
-// spreading a warp's accesses over the banks); `sync` makes the writes of all N2 threads
-// visible (a warp or block barrier, whichever spans them).
-template <int N, bool INV, class Sync>
-__device__ __forceinline__ void fft_dist(double (&xr)[Split<N>::N1], double (&xi)[Split<N>::N1], int t,
-                                         const double2* w, double* xre, double* xim, Sync sync) {
-    constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-    dft_reg<N1, N, INV>(xr, xi, w);
-#pragma unroll
-    for (int k1 = 0; k1 < N1; k1++) {
-        const double2 tw = w[(t * k1) & (N - 1)];
-        const double c = tw.x, sn = INV ? -tw.y : tw.y;
-        const double r = xr[k1], i = xi[k1];
-        xre[k1 * (N2 + 1) + t] = k1 == 0 ? r : fma(r, c, -i * sn);
-        xim[k1 * (N2 + 1) + t] = k1 == 0 ? i : fma(r, sn, i * c);
-    }
-    sync();
-#pragma unroll
-    for (int a = 0; a < N1 / N2; a++) {
-        double yr[N2], yi[N2];
-        const int k1 = t + N2 * a;
-#pragma unroll
-        for (int n2 = 0; n2 < N2; n2++) {
-            yr[n2] = xre[k1 * (N2 + 1) + n2];
-            yi[n2] = xim[k1 * (N2 + 1) + n2];
-        }
-        dft_reg<N2, N, INV>(yr, yi, w);
-#pragma unroll
-        for (int k2 = 0; k2 < N2; k2++) {
-            xr[a * N2 + k2] = yr[k2];
-            xi[a * N2 + k2] = yi[k2];
-        }
-    }
-    sync();  // the buffer is free again
-}
+// One sequence's transform by its N2 threads (t = this thread's rank). `sync` makes the
+// writes of all of them visible. (xre, xim) is the sequence's exchange buffer: N1 rows of
+// N2 + 1 doubles, the pad spreading a warp's accesses over the banks.
+template <int N1, int N2>
+struct Dist {
+    static constexpr int N = N1 * N2, A = (N1 + N2 - 1) / N2;  // A: k1 per thread at most
+    // 4 modulo 16 doubles: consecutive sequences' buffers start 8 banks apart
+    static constexpr int kLen = (N1 * (N2 + 1) + 11) / 16 * 16 + 4;
 
-// Index, in the sequence, of register q after fft_dist (thread t): (t + N2 a) + N1 k2 for
-// q = a N2 + k2. It is also the input index n1 N2 + t of register n1 = q' for the inverse:
-// X[m] with m = t + N2 n1' sits in register q where n1' = a + (N1 / N2) k2.
-template <int N>
-__device__ __forceinline__ int out_index(int t, int q) {
-    constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-    return (t + N2 * (q / N2)) + N1 * (q % N2);
-}
+    // in: xr[n1] = x[n1 N2 + t]; out: yr[a][k2] = X[(t + N2 a) + N1 k2] where t + N2 a < N1
+    template <bool INV, class Sync>
+    __device__ static __forceinline__ void run(double (&xr)[N1], double (&xi)[N1], double (&yr)[A][N2], double (&yi)[A][N2],
+                                               int t, const double2* w, double* xre, double* xim, Sync sync) {
+        dft_reg<N1, N, INV>(xr, xi, w);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) {
+            const double2 tw = w[t * k1];  // t k1 < N1 N2
+            const double c = tw.x, sn = INV ? -tw.y : tw.y;
+            const double r = xr[k1], i = xi[k1];
+            xre[k1 * (N2 + 1) + t] = k1 == 0 ? r : fma(r, c, -i * sn);
+            xim[k1 * (N2 + 1) + t] = k1 == 0 ? i : fma(r, sn, i * c);
+        }
+        sync();
+#pragma unroll
+        for (int a = 0; a < A; a++) {
+            const int k1 = min(t + N2 * a, N1 - 1);
+#pragma unroll
+            for (int n2 = 0; n2 < N2; n2++) {
+                yr[a][n2] = xre[k1 * (N2 + 1) + n2];
+                yi[a][n2] = xim[k1 * (N2 + 1) + n2];
+            }
+            dft_reg<N2, N, INV>(yr[a], yi[a], w);
+        }
+        sync();  // the buffer is free again
+    }
+    // The inverse from run()'s output: the same steps backwards.
+    template <class Sync>
+    __device__ static __forceinline__ void back(double (&yr)[A][N2], double (&yi)[A][N2], double (&xr)[N1], double (&xi)[N1],
+                                                int t, const double2* w, double* xre, double* xim, Sync sync) {
+#pragma unroll
+        for (int a = 0; a < A; a++) {
+            const int k1 = t + N2 * a;
+            if (k1 >= N1) continue;
+            dft_reg<N2, N, true>(yr[a], yi[a], w);
+#pragma unroll
+            for (int n2 = 0; n2 < N2; n2++) {
+                const double2 tw = w[n2 * k1];
+                const double c = tw.x, sn = -tw.y, r = yr[a][n2], i = yi[a][n2];
+                xre[k1 * (N2 + 1) + n2] = n2 == 0 ? r : fma(r, c, -i * sn);
+                xim[k1 * (N2 + 1) + n2] = n2 == 0 ? i : fma(r, sn, i * c);
+            }
+        }
+        sync();
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) {
+            xr[k1] = xre[k1 * (N2 + 1) + t];
+            xi[k1] = xim[k1 * (N2 + 1) + t];
+        }
+        dft_reg<N1, N, true>(xr, xi, w);
+    }
+};
 
 constexpr int kRegRows = 8;  // sequences per CTA in the row and column passes
 
+// The barrier among a row's threads: they lie in one warp where N2 divides it.
+template <int N2>
+__device__ __forceinline__ void row_sync() {
+    if (32 % N2 == 0) __syncwarp();
+    else __syncthreads();
+}
+
 // pass K forward: real rows of N (q) -> spectrum rows of N/2+1; a CTA of kRegRows x N2
-// threads takes kRegRows consecutive rows, thread (r, t) = r N2 + t (a row's threads in one
-// warp, reading consecutive values)
-template <int N>
-__global__ void __launch_bounds__(kRegRows * Split<N>::N2) k_rows_fwd(const double* __restrict__ in,
-                                                                    double2* __restrict__ spec,
-                                                                    const double2* __restrict__ W, long rows) {
-    constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, NH = N / 2 + 1;
+// threads takes kRegRows consecutive rows, thread (r, t) = r N2 + t, reading consecutive
+// values
+template <int N1, int N2>
+__global__ void __launch_bounds__(kRegRows * N2) k_rows_fwd(const double* __restrict__ in, double2* __restrict__ spec,
+                                                            const double2* __restrict__ W, long rows) {
+    using D = Dist<N1, N2>;
+    constexpr int N = D::N, NH = N / 2 + 1;
     __shared__ double2 w[N];
-    __shared__ double xre[kRegRows][XchLen<N>], xim[kRegRows][XchLen<N>];
+    __shared__ double xre[kRegRows][D::kLen], xim[kRegRows][D::kLen];
     for (int m = threadIdx.x; m < N; m += blockDim.x) w[m] = W[m];
     __syncthreads();
     const int r = threadIdx.x / N2, t = threadIdx.x % N2;
     const long row = (long)blockIdx.x * kRegRows + r;
     const bool live = row < rows;
-    double xr[N1], xi[N1];
+    double xr[N1], xi[N1], yr[D::A][N2], yi[D::A][N2];
 #pragma unroll
     for (int n1 = 0; n1 < N1; n1++) {
         xr[n1] = live ? in[row * N + n1 * N2 + t] : 0.0;
         xi[n1] = 0.0;
     }
-    fft_dist<N, false>(xr, xi, t, w, xre[r], xim[r], [] { __syncwarp(); });
+    D::template run<false>(xr, xi, yr, yi, t, w, xre[r], xim[r], row_sync<N2>);
     if (!live) return;
 #pragma unroll
-    for (int q = 0; q < N1; q++) {
-        const int m = out_index<N>(t, q);
-        if (m < NH) spec[row * NH + m] = make_double2(xr[q], xi[q]);
+    for (int a = 0; a < D::A; a++) {
+        const int k1 = t + N2 * a;
+        if (k1 >= N1) continue;
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++) {
+            const int m = k1 + N1 * k2;
+            if (m < NH) spec[row * NH + m] = make_double2(yr[a][k2], yi[a][k2]);
+        }
     }
 }
 
 // pass K': spectrum rows (Hermitian, N/2+1 stored) -> real rows of N
-template <int N>
-__global__ void __launch_bounds__(kRegRows * Split<N>::N2) k_rows_inv(const double2* __restrict__ spec,
-                                                                    double* __restrict__ out,
-                                                                    const double2* __restrict__ W, long rows) {
-    constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, NH = N / 2 + 1;
+template <int N1, int N2>
+__global__ void __launch_bounds__(kRegRows * N2) k_rows_inv(const double2* __restrict__ spec, double* __restrict__ out,
+                                                            const double2* __restrict__ W, long rows) {
+    using D = Dist<N1, N2>;
+    constexpr int N = D::N, NH = N / 2 + 1;
     __shared__ double2 w[N];
-    __shared__ double xre[kRegRows][XchLen<N>], xim[kRegRows][XchLen<N>];
+    __shared__ double xre[kRegRows][D::kLen], xim[kRegRows][D::kLen];
     for (int m = threadIdx.x; m < N; m += blockDim.x) w[m] = W[m];
     __syncthreads();
     const int r = threadIdx.x / N2, t = threadIdx.x % N2;
     const long row = (long)blockIdx.x * kRegRows + r;
     const bool live = row < rows;
-    double xr[N1], xi[N1];
+    double xr[N1], xi[N1], yr[D::A][N2], yi[D::A][N2];
 #pragma unroll
     for (int n1 = 0; n1 < N1; n1++) {
         const int m = n1 * N2 + t;
         double2 v = make_double2(0.0, 0.0);
         if (live) {
-            if (m < NH) v = spec[row * NH + m];
-            else {
-                v = spec[row * NH + (N - m)];
-                v.y = -v.y;
-            }
+            v = spec[row * NH + (m < NH ? m : N - m)];
+            if (m >= NH) v.y = -v.y;
         }
         xr[n1] = v.x;
         xi[n1] = v.y;
     }
-    fft_dist<N, true>(xr, xi, t, w, xre[r], xim[r], [] { __syncwarp(); });
+    D::template run<true>(xr, xi, yr, yi, t, w, xre[r], xim[r], row_sync<N2>);
     if (!live) return;
 #pragma unroll
-    for (int q = 0; q < N1; q++) out[row * N + out_index<N>(t, q)] = xr[q];
+    for (int a = 0; a < D::A; a++) {
+        const int k1 = t + N2 * a;
+        if (k1 >= N1) continue;
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++) out[row * N + k1 + N1 * k2] = yr[a][k2];
+    }
 }
 
 // passes J / I: columns of the spectrum (MODE 0 forward along j, 1 inverse along j, 2
 // forward along i, ig2 multiply, inverse along i). A CTA takes kRegRows consecutive kh of
 // one i (MODE 0/1) or one j (MODE 2); thread (t, f) = t kRegRows + f, so a warp reads whole
 // 128-byte runs of kh; a column's threads span warps and exchange through the block.
-template <int N, int MODE>
-__global__ void __launch_bounds__(kRegRows * Split<N>::N2) k_cols_reg(double2* __restrict__ spec,
-                                                                    const double2* __restrict__ W,
-                                                                    const double* __restrict__ freq,
-                                                                    const double* __restrict__ rfreq, double cst) {
-    constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, NH = N / 2 + 1;
+template <int N1, int N2, int MODE>
+__global__ void __launch_bounds__(kRegRows * N2) k_cols_reg(double2* __restrict__ spec, const double2* __restrict__ W,
+                                                            const double* __restrict__ freq,
+                                                            const double* __restrict__ rfreq, double cst) {
+    using D = Dist<N1, N2>;
+    constexpr int N = D::N, NH = N / 2 + 1;
     constexpr int NT = (NH + kRegRows - 1) / kRegRows;
     __shared__ double2 w[N];
-    __shared__ double xre[kRegRows][XchLen<N>], xim[kRegRows][XchLen<N>];
+    __shared__ double xre[kRegRows][D::kLen], xim[kRegRows][D::kLen];
     for (int m = threadIdx.x; m < N; m += blockDim.x) w[m] = W[m];
     __syncthreads();
     const int t = threadIdx.x / kRegRows, f = threadIdx.x % kRegRows;
@@ -461,7 +502,7 @@ __global__ void __launch_bounds__(kRegRows * Split<N>::N2) k_cols_reg(double2* _
     // element e of the column: (i = fixed, j = e) for MODE 0/1, (i = e, j = fixed) for MODE 2
     auto addr = [&](int e) -> long { return MODE == 2 ? (long)e * nnh + (long)fixed * NH + kh
                                                       : (long)fixed * nnh + (long)e * NH + kh; };
-    double xr[N1], xi[N1];
+    double xr[N1], xi[N1], yr[D::A][N2], yi[D::A][N2];
 #pragma unroll
     for (int n1 = 0; n1 < N1; n1++) {
         const double2 v = live ? spec[addr(n1 * N2 + t)] : make_double2(0.0, 0.0);
@@ -469,60 +510,85 @@ __global__ void __launch_bounds__(kRegRows * Split<N>::N2) k_cols_reg(double2* _
         xi[n1] = v.y;
     }
     auto bar = [] { __syncthreads(); };
-    if (MODE == 1)
-        fft_dist<N, true>(xr, xi, t, w, xre[f], xim[f], bar);
-    else
-        fft_dist<N, false>(xr, xi, t, w, xre[f], xim[f], bar);
+    D::template run<MODE == 1>(xr, xi, yr, yi, t, w, xre[f], xim[f], bar);
     if (MODE == 2) {
         // ig2(i, j, kh) = cst / ((freq_i^2 + freq_j^2) + rfreq_kh^2 + 1e-10), DC untouched
         const double fj = freq[fixed], rk = live ? rfreq[kh] : 0.0;
-        double yr[N1], yi[N1];
 #pragma unroll
-        for (int q = 0; q < N1; q++) {
-            const int e = out_index<N>(t, q);
-            double g = 1.0;
-            if (!(e == 0 && fixed == 0 && kh == 0)) {
-                const double fi = freq[e];
-                const double f1 = fi * fi;
-                const double f2 = f1 + fj * fj;
-                g = cst / (f2 + rk * rk + 1E-10);
+        for (int a = 0; a < D::A; a++) {
+            const int k1 = min(t + N2 * a, N1 - 1);
+#pragma unroll
+            for (int k2 = 0; k2 < N2; k2++) {
+                const int e = k1 + N1 * k2;
+                double g = 1.0;
+                if (!(e == 0 && fixed == 0 && kh == 0)) {
+                    const double fi = freq[e];
+                    const double f1 = fi * fi;
+                    const double f2 = f1 + fj * fj;
+                    g = cst / (f2 + rk * rk + 1E-10);
+                }
+                yr[a][k2] *= g;
+                yi[a][k2] *= g;
             }
-            // register q holds X[e], e - t = N2 (q / N2) + N1 (q % N2): the inverse's input
-            // n1' = (e - t) / N2
-            const int n1p = q / N2 + (N1 / N2) * (q % N2);
-            yr[n1p] = xr[q] * g;
-            yi[n1p] = xi[q] * g;
         }
-        fft_dist<N, true>(yr, yi, t, w, xre[f], xim[f], bar);
+        D::back(yr, yi, xr, xi, t, w, xre[f], xim[f], bar);
+        if (!live) return;
 #pragma unroll
-        for (int q = 0; q < N1; q++) {
-            xr[q] = yr[q];
-            xi[q] = yi[q];
-        }
+        for (int n1 = 0; n1 < N1; n1++) spec[addr(n1 * N2 + t)] = make_double2(xr[n1], xi[n1]);
+        return;
     }
     if (!live) return;
 #pragma unroll
-    for (int q = 0; q < N1; q++) spec[addr(out_index<N>(t, q))] = make_double2(xr[q], xi[q]);
+    for (int a = 0; a < D::A; a++) {
+        const int k1 = t + N2 * a;
+        if (k1 >= N1) continue;
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++) spec[addr(k1 + N1 * k2)] = make_double2(yr[a][k2], yi[a][k2]);
+    }
 }
 
-template <int N>
+template <int N1, int N2>
 void solve_reg(const double* q, double* phi, double2* spec, const double2* W, const double* freq, const double* rfreq,
                double cst, cudaStream_t s) {
-    constexpr int T = kRegRows * Split<N>::N2, NH = N / 2 + 1;
+    constexpr int N = N1 * N2, T = kRegRows * N2, NH = N / 2 + 1;
     constexpr int NT = (NH + kRegRows - 1) / kRegRows;
     const long rows = (long)N * N;
     const int rblocks = (int)((rows + kRegRows - 1) / kRegRows);
     count_launch();
-    k_rows_fwd<N><<<rblocks, T, 0, s>>>(q, spec, W, rows);
+    k_rows_fwd<N1, N2><<<rblocks, T, 0, s>>>(q, spec, W, rows);
     count_launch();
-    k_cols_reg<N, 0><<<N * NT, T, 0, s>>>(spec, W, freq, rfreq, cst);
+    k_cols_reg<N1, N2, 0><<<N * NT, T, 0, s>>>(spec, W, freq, rfreq, cst);
     count_launch();
-    k_cols_reg<N, 2><<<N * NT, T, 0, s>>>(spec, W, freq, rfreq, cst);
+    k_cols_reg<N1, N2, 2><<<N * NT, T, 0, s>>>(spec, W, freq, rfreq, cst);
     count_launch();
-    k_cols_reg<N, 1><<<N * NT, T, 0, s>>>(spec, W, freq, rfreq, cst);
+    k_cols_reg<N1, N2, 1><<<N * NT, T, 0, s>>>(spec, W, freq, rfreq, cst);
     count_launch();
-    k_rows_inv<N><<<rblocks, T, 0, s>>>(spec, phi, W, rows);
+    k_rows_inv<N1, N2><<<rblocks, T, 0, s>>>(spec, phi, W, rows);
     MZB_CHECK(cudaGetLastError());
+}
+
+using RegSolver = void (*)(const double*, double*, double2*, const double2*, const double*, const double*, double,
+                           cudaStream_t);
+// The sizes worked in registers: the products of two factors of 4 .. 18 nearest each other,
+// up to 256 (one that is missing here, or larger, takes the Stockham kernels).
+RegSolver reg_solver(int n) {
+    switch (n) {
+    case 32: return solve_reg<8, 4>;
+    case 36: return solve_reg<6, 6>;
+    case 48: return solve_reg<8, 6>;
+    case 54: return solve_reg<9, 6>;
+    case 64: return solve_reg<8, 8>;
+    case 72: return solve_reg<9, 8>;
+    case 96: return solve_reg<12, 8>;
+    case 108: return solve_reg<12, 9>;
+    case 128: return solve_reg<16, 8>;
+    case 144: return solve_reg<12, 12>;
+    case 162: return solve_reg<18, 9>;
+    case 192: return solve_reg<16, 12>;
+    case 216: return solve_reg<18, 12>;
+    case 256: return solve_reg<16, 16>;
+    default: return nullptr;
+    }
 }
 
 }  // namespace
@@ -567,9 +633,7 @@ void FftPoisson::release() {
 void FftPoisson::solve(const double* q, double* phi, cudaStream_t s) const {
     // constant = 4 pi / (h h h) / (n n n)   (grid_fft.c:105)
     const double cst0 = 4 * kPi / (h * h * h) / (double)(n * n * n);
-    if (n == 256) return solve_reg<256>(q, phi, spec, W, freq, rfreq, cst0, s);
-    if (n == 128) return solve_reg<128>(q, phi, spec, W, freq, rfreq, cst0, s);
-    if (n == 64) return solve_reg<64>(q, phi, spec, W, freq, rfreq, cst0, s);
+    if (const RegSolver reg = reg_solver(n)) return reg(q, phi, spec, W, freq, rfreq, cst0, s);
     const Radices rd = plan_radices(n);
     const long rows = (long)n * n;
     const int rblocks = (int)((rows + kRowsPerBlock - 1) / kRowsPerBlock);
@@ -577,8 +641,7 @@ void FftPoisson::solve(const double* q, double* phi, cudaStream_t s) const {
     const int cblocks = n * ntk;
     const size_t rows_smem = (2 * n + 4 * kRowsPerBlock * n) * sizeof(double);
     const size_t cols_smem = (2 * n + 4 * kColsPerBlock * n) * sizeof(double);
-    // constant = 4 pi / (h h h) / (n n n)   (grid_fft.c:105)
-    const double cst = 4 * kPi / (h * h * h) / (double)(n * n * n);
+    const double cst = cst0;
     count_launch();
     k_pass_k_fwd<<<rblocks, kFftThreads, rows_smem, s>>>(q, spec, W, n, rd);
     count_launch();

@@ -295,7 +295,7 @@ void ensure_mixed_levels(GridState& G) {
 
 void free_particles(ParticleDev& P) {
     dfree(P.types); dfree(P.pos); dfree(P.vel); dfree(P.fe); dfree(P.fn); dfree(P.ft);
-    dfree(P.mass); dfree(P.chg); dfree(P.tab); dfree(P.base);
+    dfree(P.mass); dfree(P.chg); dfree(P.tab); dfree(P.base); dfree(P.wgt);
     dfree(P.tile_count); dfree(P.tile_start); dfree(P.tile_fill); dfree(P.tile_ions); dfree(P.tile_part);
     dfree(P.cell_of); dfree(P.cell_count); dfree(P.cell_start); dfree(P.cell_fill);
     dfree(P.cell_ions); dfree(P.srank); dfree(P.spos); dfree(P.stype); dfree(P.fpart);
@@ -753,6 +753,7 @@ void solver_initialize_particles(int n, int n_typ, double L, double h, int n_p, 
     P.mass = dalloc<double>(n_p);
     P.chg = dalloc<double>(n_p);
     P.base = dalloc<int32_t>(v3);
+    if (cas_type != CAS_CIC) P.wgt = dalloc<double>((size_t)12 * n_p);
     if (n_p > 0) {
         upload(P.types, types, sizeof(int32_t) * n_p);
         upload(P.pos, pos, sizeof(double) * v3);

@@ -261,12 +261,32 @@ __device__ __forceinline__ void k_spread_bin_body(const ParticleDev& P, int n, d
         const int tile = ((b[0] / kTileI) * P.ntj + b[1] / kTileJ) * P.ntk + b[2] / kTileK;
         atomicAdd(&P.tile_count[tile], 1);
         const double L = n * h, q = P.chg[p];
-        for (int o = 0; o < stencil_size<CAS>(); o++) {
-            int a, bb, e;
-            stencil_point<CAS>(o, b, n, a, bb, e);
-            double w = w_cas<CAS>(P.pos[3 * p] - a * h, L, h) * w_cas<CAS>(P.pos[3 * p + 1] - bb * h, L, h);
-            w = w * w_cas<CAS>(P.pos[3 * p + 2] - e * h, L, h);
-            u += q * w;
+        if (CAS == CAS_CIC) {
+            for (int o = 0; o < stencil_size<CAS>(); o++) {
+                int a, bb, e;
+                stencil_point<CAS>(o, b, n, a, bb, e);
+                double w = w_cas<CAS>(P.pos[3 * p] - a * h, L, h) * w_cas<CAS>(P.pos[3 * p + 1] - bb * h, L, h);
+                w = w * w_cas<CAS>(P.pos[3 * p + 2] - e * h, L, h);
+                u += q * w;
+            }
+        } else {
+            // the twelve one-dimensional weights once (they carry two divisions each), kept
+            // for the tiles; the products and their order are the 64 points' own
+            double w1[3][4];
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+#pragma unroll
+                for (int o = 0; o < 4; o++) {
+                    const int g = (b[d] + o - 1 + n) % n;
+                    w1[d][o] = w_cas<CAS>(P.pos[3 * p + d] - g * h, L, h);
+                    P.wgt[(size_t)(4 * d + o) * P.np + p] = w1[d][o];
+                }
+#pragma unroll
+            for (int o = 0; o < 64; o++) {
+                double w = w1[0][o / 16] * w1[1][(o / 4) % 4];
+                w = w * w1[2][o % 4];
+                u += q * w;
+            }
         }
     }
     __shared__ double sh[4 * 32];
@@ -287,15 +307,6 @@ __device__ __forceinline__ void k_spread_fill_body(const ParticleDev& P, int bx)
 }
 __global__ void k_spread_fill(ParticleDev P) { k_spread_fill_body(P, blockIdx.x); }
 
-// Is grid index g one of the stencil's indices along an axis with base index b (wrapped)?
-// CIC: b, b+1; splines: b-1 .. b+2 (particles.c:297-385).
-template <int CAS>
-__device__ __forceinline__ bool in_stencil(int g, int b, int n) {
-    if (CAS == CAS_CIC) return g == b || g == (b + 1 == n ? 0 : b + 1);
-    const int d = g - b + 1;
-    return (d >= 0 && d <= 3) || (d + n >= 0 && d + n <= 3) || (d - n >= 0 && d - n <= 3);
-}
-
 // Spline spreading (CIC takes k_spread_ions below). One warp per tile (grid-stride over
 // warps): gather the ions whose stencil can reach the tile (base cell in this tile or the
 // 7 tiles below it for CIC, whose +1 corners reach up; in the 27 tiles around it for the
@@ -303,9 +314,11 @@ __device__ __forceinline__ bool in_stencil(int g, int b, int n) {
 // ion index (beyond kTileCap candidates, take them in the same order by repeated warp
 // minima over the source tiles' lists instead), and let every lane sum the contributions of its TI x TJ points (one k column)
 // over those ions in ascending ion order -- for each point the order of the reference's
-// serial scatter (charges.c:123-141), with the same weight expression -- then write the
+// serial scatter (charges.c:123-141), with the weights k_spread_bin formed -- then write the
 // tile, zeros included, 32 consecutive k per store. q is written once; no atomics touch
-// it, and the warps of a CTA never wait on one another.
+// it, and the warps of a CTA never wait on one another. Forming the weights here, per
+// point, was most of the time (144^3, 2662 ions, cubic: 91 us against 20; in
+// k_spread_bin, per stencil point, 64 us against 6.5).
 constexpr int kSpreadWarps = 4;
 constexpr int kSpreadStage = 32;  // staged candidates per round (one per lane)
 
@@ -315,19 +328,18 @@ __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_tiles(ParticleDev 
     constexpr int NSRC = CAS == CAS_CIC ? 8 : 27;
     __shared__ int cand_all[kSpreadWarps][kTileCap];
     __shared__ int sorted_all[kSpreadWarps][kTileCap];
-    __shared__ double spos_all[kSpreadWarps][kSpreadStage][4];  // x, y, z, charge (rank order)
+    __shared__ double swgt_all[kSpreadWarps][kSpreadStage][13];  // the 12 weights, charge (rank order)
     __shared__ int sbase_all[kSpreadWarps][kSpreadStage][3];
     __shared__ int srcs_all[kSpreadWarps][32];
     __shared__ int lfirst_all[kSpreadWarps][32], lcnt_all[kSpreadWarps][32];  // source lists (overflow path)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int* cand = cand_all[w];
     int* sorted = sorted_all[w];
-    double (*spos)[4] = spos_all[w];
+    double (*swgt)[13] = swgt_all[w];
     int (*sbase)[3] = sbase_all[w];
     int* srcs = srcs_all[w];
     int* lfirst = lfirst_all[w];
     int* lcnt = lcnt_all[w];
-    const double L = n * h;
     const long n2 = (long)n * n;
     const long nwarps = (long)gridDim.x * kSpreadWarps;
     for (long tile = (long)blockIdx.x * kSpreadWarps + w; tile < P.ntiles; tile += nwarps) {
@@ -374,33 +386,38 @@ __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_tiles(ParticleDev 
         // round's cn ions, in lane order, to its points
         auto stage_and_add = [&](int p, int cn) {
             if (p >= 0) {
-                spos[lane][0] = P.pos[3 * p];
-                spos[lane][1] = P.pos[3 * p + 1];
-                spos[lane][2] = P.pos[3 * p + 2];
-                spos[lane][3] = P.chg[p];
+#pragma unroll
+                for (int o = 0; o < 12; o++) swgt[lane][o] = P.wgt[(size_t)o * P.np + p];
+                swgt[lane][12] = P.chg[p];
                 sbase[lane][0] = P.base[3 * p];
                 sbase[lane][1] = P.base[3 * p + 1];
                 sbase[lane][2] = P.base[3 * p + 2];
             }
             __syncwarp();
-            if (k < n) {
-                for (int x = 0; x < cn; x++) {
-                    if (!in_stencil<CAS>(k, sbase[x][2], n)) continue;
-                    const double zk = w_cas<CAS>(spos[x][2] - k * h, L, h);
-                    const double cq = spos[x][3];
+            for (int x = 0; x < cn; x++) {
+                // offset of grid index g in the ion's stencil (0 .. 3), wrapped (n >= 4)
+                auto offset = [&](int g, int b) {
+                    const int d = g - b + 1;
+                    return d < 0 ? d + n : d >= n ? d - n : d;
+                };
+                const int da = offset(i0, sbase[x][0]), db = offset(j0, sbase[x][1]);
+                // the tile's rows the stencil meets; none for most candidates
+                if ((da > 3 && da + kTileI <= n) || (db > 3 && db + kTileJ <= n)) continue;
+                const int dk = offset(k, sbase[x][2]);
+                if (k >= n || dk > 3) continue;
+                const double zk = swgt[x][8 + dk], cq = swgt[x][12];
 #pragma unroll
-                    for (int a = 0; a < kTileI; a++) {
-                        const int i = i0 + a;
-                        if (i >= n || !in_stencil<CAS>(i, sbase[x][0], n)) continue;
-                        const double wx = w_cas<CAS>(spos[x][0] - i * h, L, h);
+                for (int a = 0; a < kTileI; a++) {
+                    const int di = offset(i0 + a, sbase[x][0]);
+                    if (i0 + a >= n || di > 3) continue;
+                    const double wx = swgt[x][di];
 #pragma unroll
-                        for (int r = 0; r < kTileJ; r++) {
-                            const int j = j0 + r;
-                            if (j < n && in_stencil<CAS>(j, sbase[x][1], n)) {
-                                double wgt = wx * w_cas<CAS>(spos[x][1] - j * h, L, h);
-                                wgt = wgt * zk;
-                                acc[a][r] += cq * wgt;
-                            }
+                    for (int r = 0; r < kTileJ; r++) {
+                        const int dj = offset(j0 + r, sbase[x][1]);
+                        if (j0 + r < n && dj <= 3) {
+                            double wgt = wx * swgt[x][4 + dj];
+                            wgt = wgt * zk;
+                            acc[a][r] += cq * wgt;
                         }
                     }
                 }
@@ -668,13 +685,28 @@ __device__ __forceinline__ void k_field_forces_body(const ParticleDev& P, const 
     const int* b = P.base + 3 * p;
     const double px = P.pos[3 * p], py = P.pos[3 * p + 1], pz = P.pos[3 * p + 2], chg = P.chg[p];
     double tx[T], ty[T], tz[T];
+    // splines: the group's lanes form the twelve one-dimensional weights (x offsets in lanes
+    // 0 .. 3, y in lanes 4 .. 7, z in both) and hand them round by shuffles
+    double wxy = 0.0, wz = 0.0;
+    if (CAS != CAS_CIC) {
+        const int o = (sub & 3) - 1, g = ((sub < 4 ? b[0] : b[1]) + o + n) % n;
+        wxy = w_cas<CAS>((sub < 4 ? px : py) - g * h, L, h);
+        wz = w_cas<CAS>(pz - (b[2] + o + n) % n * h, L, h);
+    }
 #pragma unroll
     for (int u = 0; u < T; u++) {
         int i, j, k;
         stencil_point<CAS>(u * kForceLanes + sub, b, n, i, j, k);
-        double qc = chg * w_cas<CAS>(px - i * h, L, h);
-        qc = qc * w_cas<CAS>(py - j * h, L, h);
-        qc = qc * w_cas<CAS>(pz - k * h, L, h);
+        double qc;
+        if (CAS == CAS_CIC) {
+            qc = chg * w_cas<CAS>(px - i * h, L, h);
+            qc = qc * w_cas<CAS>(py - j * h, L, h);
+            qc = qc * w_cas<CAS>(pz - k * h, L, h);
+        } else {  // point u 8 + sub: offsets u / 2, (2 u + sub / 4) % 4, sub % 4 (its own wz)
+            qc = chg * __shfl_sync(gmask, wxy, g0 + u / 2);
+            qc = qc * __shfl_sync(gmask, wxy, g0 + 4 + ((2 * u + sub / 4) & 3));
+            qc = qc * wz;
+        }
         const long i0 = i * n2, j0 = (long)j * n;
         const long ip = (long)wrap_inc(i, n) * n2, im = (long)wrap_dec(i, n) * n2;
         const long jp = (long)wrap_inc(j, n) * n, jm = (long)wrap_dec(j, n) * n;

@@ -39,6 +39,7 @@ struct ParticleDev {
     double* tab = nullptr;   // [ntyp*ntyp][kPairConsts] pair-potential constants per type pair
     int32_t* base = nullptr; // [np][3] base cell floor(pos/h) (wrapped)
     int cas = CAS_CIC;       // charge assignment scheme
+    double* wgt = nullptr;   // [12][np] spline weights of the last spreading: x, y, z offsets -1 .. 2 (null for CIC)
     // the charge grid whose only nonzeros are the CIC corners of `base` (left by the last
     // CIC spreading into it), or null: the next CIC spreading into it zeroes those corners
     // instead of the whole grid

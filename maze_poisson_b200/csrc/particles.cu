@@ -1171,7 +1171,7 @@ void stage_blocks(const StageArgs& a, int* c) {
     c[SK_TF_TF] = has && P.pot == POT_TF ? P.tf_nst : 0;
     c[SK_TF_LJ] = has && P.pot == POT_LJ ? P.tf_nst : 0;
     c[SK_TF_SC] = has && P.pot == POT_SC ? P.tf_nst : 0;
-    c[SK_TFG] = has ? cdiv(32 * nblk32, 128) : 0;
+    c[SK_TFG] = has ? nblk32 : 0;
     c[SK_TFE] = 1;
     c[SK_TOT] = has ? cdiv(3 * np, 256) : 0;
 }

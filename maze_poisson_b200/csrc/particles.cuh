@@ -64,13 +64,14 @@ struct ParticleDev {
     int32_t* srank = nullptr;        // [np] position of ion p in cell order
     double* spos = nullptr;          // [np][3] positions in cell order
     int32_t* stype = nullptr;        // [np]
-    // pair-force plan (tf_forces.cu): super-tiles of 8 x 8 blocks of 32 cell-ordered ions
+    // pair-force plan (tf_forces.cu): super-tiles of tf_sb x tf_sb blocks of 32 cell-ordered ions
+    int tf_sb = 0;                   // 8, 4 or 2
     int tf_nst = 0;                  // super-tiles (CTAs of the pair-force kernel)
     int* tf_st = nullptr;            // [tf_nst][2] (I super-block, J super-block)
     int* tf_gstart = nullptr;        // [nblk + 1] gather-list offsets per block
     int* tf_gent = nullptr;          // gather entries (super-tile << 4 | side << 3 | slot)
     double* tf_box = nullptr;        // [nblk][6] bounding boxes of the blocks
-    double* fpart = nullptr;         // [tf_nst][2][8][32][3] force partials
+    double* fpart = nullptr;         // [tf_nst][2][tf_sb][32][3] force partials
     double* epart = nullptr;         // [tf_nst] energy partials
 
     // Poisson-Boltzmann (solver_initialize_particles_pois_boltz, particles.c:111-127);

@@ -10,41 +10,67 @@
 // reference, which uses glibc exp/pow.
 //
 // Layout. Ions are sorted by linked cell (particles.cu), cut into blocks of 32 and the
-// blocks into super-blocks of 8 (256 ions). A CTA of 8 warps takes one super-block pair
-// (SI, SJ) of a half shell (SJ = SI + d, d = 0 .. nsb/2, the middle distance only once):
-// warp w owns block I = 8 SI + w -- one ion per lane, its forces in registers -- and
-// walks the J blocks of SJ; in step s (0..15) lane l pairs its ion with ions (l + s) and
-// (l + s + 16) mod 32 of the J block, two independent chains, so the 32 lanes touch 32
-// distinct J ions at a time and add the reactions into a warp-private shared array
-// (structure of arrays, conflict-free) without atomics, with a __syncwarp between the two
-// halves. On the diagonal super-tile each unordered block pair is taken once (and each
-// pair inside a block once, 16 steps of one partner). A tile whose bounding
-// boxes are farther apart than r_cut (minimum image, 1e-9 relative margin) is skipped;
-// pruning is off when a coordinate lies outside [0, L). Inside a tile, a step in which no
-// lane's two partners lie inside r_cut skips the pair terms (a warp vote). 1/r is an FP32
-// seed refined by two FP64 Newton steps; types sit in the shared position arrays as integer
-// bits; the pair-constant rows have an odd stride (no bank conflicts between type pairs).
+// blocks into super-blocks of SB blocks. A CTA of 8 warps takes one super-block pair
+// (SI, SJ) of a half shell (SJ = SI + d, d = 0 .. nsb/2, the middle distance only once). A
+// warp holds two neighbouring I blocks, one ion of each per lane with its force in registers;
+// the 16 / SB warps of an I pair split the J blocks of SJ, then the 32 steps of a block, among
+// them. In step s lane l pairs its two ions with ion (l + s) mod 32 of the J block: two
+// independent chains that share one load of the partner and one update of its reaction, kept
+// in a warp-private shared array (structure of arrays, conflict-free) without atomics, with a
+// __syncwarp per step. SB is the largest of 8, 4, 2 that still gives kTfMinCtas CTAs
+// (tf_plan): with SB = 8 throughout, 250 ions were one CTA and 2000 ions 36.
+// On the diagonal super-tile each unordered block pair is taken once (and each pair inside a
+// block once: steps 1 .. 15 and half of step 16). A tile whose bounding boxes are farther
+// apart than r_cut (minimum image, 1e-9 relative margin) is left out; pruning is off when a
+// coordinate lies outside [0, L). A step in which no lane's pair lies inside r_cut skips the
+// pair terms (a warp vote).
 //
-// Determinism. Registers and warp arrays accumulate in step order; the warps' J partials
-// are summed in warp order; each ion's force is the sum of its super-tile partials in a
+// Cost. At 16000 ions the kernel was bound by shared-memory wavefronts (68 %, FP64 pipe 49 %,
+// issue 60 %): a pair loaded its partner, seven constants and the reaction, 34 wavefronts for
+// 40 FP64 instructions, and a 64-bit load costs an SM four times what an FP64 instruction
+// does. So one J ion serves two I ions, a pair beyond the exponential's range reads four
+// constants in two loads, and nothing goes through the conversion pipe: the nearest image by adding and subtracting 1.5 2^52, 1/r from the hardware's FP64
+// seed and one third-order step. Pairs that are not taken read a row of zeros instead of being
+// selected out, and the exponential's branch follows both ions' other terms. At 16000 ions TF
+// 659 -> 553 us, LJ 569 -> 478 us: 84 instructions and 43 FP64 instructions a pair (104 and 43
+// with selects and single-ion lanes), FP64 pipe 60 %, issue 61 %; what is left is the latency of
+// 16 warps of two chains and the CTA's slowest warp.
+//
+// Determinism. Registers and warp arrays accumulate in step order; the warps' partials are
+// summed in warp order; each ion's force is the sum of its super-tile partials in a
 // fixed order (k_tf_gather over a host-built list), the energy the sum of the CTAs'
 // energies in CTA order.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "particles.cuh"
 
 namespace mzb {
 
-constexpr int kTfSb = 8;                  // blocks of 32 ions per super-block
-constexpr int kTfThreads = kTfSb * 32;    // one warp per I block of a super-block
-// Pair-constant table in shared memory, up to 8 types, one row of kTfTabStride doubles per
-// type pair: the odd stride puts the rows a warp reads at once (lanes of different type
-// pairs) on different banks.
-constexpr int kTfTabStride = kPairConsts + 1;
-constexpr int kTfTab = 64 * kTfTabStride;
-constexpr size_t kTfSmem =
-    sizeof(double) * (kTfTab + 2 * kTfSb * 32 * 4 + kTfSb * kTfSb * 32 * 3);
+constexpr int kTfSbMax = 8;                  // blocks of 32 ions per super-block, at most
+constexpr int kTfWarps = 8;
+constexpr int kTfThreads = kTfWarps * 32;
+constexpr int kTfResident = 2;  // CTAs per SM
+// CTAs below which smaller super-blocks pay: two waves of kTfResident on 148 SMs. SB = 8 / 4 / 2
+// at 7600 ions 187 / 163 / 222 us, at 16000 ions 548 / 577 / - us; SB = 4 / 2 at 4394 ions
+// 71 / 85 us. TF at 64 / 250 / 1024 / 2278 / 4394 / 7600 ions, SB = 8 throughout before:
+// 20 / 54 / 101 / 100 / 138 / 230 us, now 10 / 10 / 10 / 32 / 71 / 163 us.
+constexpr int kTfMinCtas = 592;
+// Pair-constant table in shared memory, up to 8 types: one row of kTfRow 16-byte slots per
+// type pair (80 bytes: the rows of four type pairs lie on different banks), and after them a
+// row of zeros, which pairs that are not taken read instead.
+constexpr int kTfRow = kPairConsts / 2 + 1;
+constexpr int kTfZero = 64 * kTfRow;
+constexpr int kTfTab = 65 * kTfRow;
+// J blocks one warp walks: SB / 2 I pairs share 8 warps
+constexpr int tf_nj(int sb) { return sb == 8 ? 4 : 1; }
+// shared memory: table, both super-blocks' positions, the warps' reaction arrays (one per J
+// block the warp walks) and I forces, both super-blocks' types
+constexpr size_t tf_smem(int sb) {
+    return sizeof(double) * (2 * kTfTab + 2 * sb * 96 + kTfWarps * tf_nj(sb) * 96 + kTfWarps * 192 + sb * 32);
+}
+constexpr size_t kTfSmem = tf_smem(8);
 
 // min-image gap along one axis between the interval [lo, hi] and the cell [c0, c0 + cl]
 __device__ __forceinline__ double axis_gap(double lo, double hi, double c0, double cl, double L) {
@@ -58,31 +84,27 @@ __device__ __forceinline__ double axis_gap(double lo, double hi, double c0, doub
     return best;
 }
 
-// Shifted-force pair force (times 1/r, to be multiplied by the separation vector) and
-// pair energy of one pair at r^2 with 1/r = ir, from the type pair's constants t.
+// Shifted-force pair force (times 1/r, to be multiplied by the separation) and energy from a
+// row of the table, without the exponential of TF (pair_exp); zero for the row of zeros. TF rows are stored as {C, D}, {alpha, beta},
+// {A, B}, {sigma, range of the exponential}, the others in the order of P.tab.
 template <int POT>
-__device__ __forceinline__ void pair_terms(const double* t, double r2, double ir, double& fr, double& vm) {
-    const double r = r2 * ir;
-    if (POT == POT_TF) {  // forces.c:112-186
-        const double a = t[0], b = t[1], c = t[2], d = t[3], sg = t[4], al = t[5], be = t[6];
-        const double ir2 = ir * ir, ir6 = ir2 * ir2 * ir2;
-        const double ir7 = ir6 * ir, ir8 = ir6 * ir2, ir9 = ir8 * ir;
-        const double ex = r2 < t[7] ? exp(b * (sg - r)) : 0.0;  // negligible beyond (tf_exp_r2_limit)
-        const double fm = b * a * ex - 6 * c * ir7 - 8 * d * ir9 - al;
-        vm = a * ex - c * ir6 - d * ir8 + al * r + be;
-        fr = fm * ir;
+__device__ __forceinline__ void pair_terms(const double2* t, double r2, double ir, double& fr, double& vm) {
+    if (POT == POT_TF) {  // forces.c:112-186: the force is B A ex - 6 C / r^7 - 8 D / r^9 - alpha
+        const double2 cd = t[0], ab = t[1];
+        const double ir2 = ir * ir, ir6 = ir2 * ir2 * ir2, g = ab.x * ir;
+        const double c6 = ir6 * cd.x, d8 = ir6 * (cd.y * ir2), s = c6 + d8;
+        fr = fma(-6.0 * ir2, fma(1.0 / 3.0, d8, s), -g);  // -(6 c6 + 8 d8) / r^2 - alpha / r
+        vm = fma(g, r2, ab.y) - s;
     } else if (POT == POT_LJ) {  // forces.c:199-271
-        const double sg = t[0], ep = t[1], al = t[2], be = t[3];
-        const double s = sg * ir, s2 = s * s, s6 = s2 * s2 * s2, s12 = s6 * s6;
-        const double fm = 4 * ep * (12 * s12 - 6 * s6) * ir - al;
-        vm = 4 * ep * (s12 - s6) + al * r + be;
-        fr = fm * ir;
+        const double2 se = t[0], ab = t[1];
+        const double s = se.x * ir, s2 = s * s, s6 = s2 * s2 * s2, s12 = s6 * s6, e4 = 4 * se.y, g = ab.x * ir;
+        fr = fma(e4 * (12 * s12 - 6 * s6), ir * ir, -g);
+        vm = fma(e4, s12 - s6, fma(g, r2, ab.y));
     } else {  // forces.c:283-337
-        const double nu = t[0], d = t[1], B = t[2], al = t[3], be = t[4];
-        const double p = pow(d * ir, nu);
-        const double fm = B * nu * p * ir - al;
-        vm = B * p + al * r + be;
-        fr = fm * ir;
+        const double2 nd = t[0], ba = t[1];
+        const double p = ba.x * pow(nd.y * ir, nd.x), g = ba.y * ir;
+        fr = fma(nd.x * p, ir * ir, -g);
+        vm = p + fma(g, r2, t[2].x);
     }
 }
 
@@ -110,230 +132,239 @@ __device__ __forceinline__ void k_tf_boxes_body(const ParticleDev& P, int bx) {
 }
 __global__ void k_tf_boxes(ParticleDev P) { k_tf_boxes_body(P, blockIdx.x); }
 
-// The ion type stored in a double slot of the shared position arrays as its integer bits
-// (read back without a conversion).
-__device__ __forceinline__ double type_bits(int t) { return __longlong_as_double((long long)t); }
-__device__ __forceinline__ int type_of(double v) { return (int)__double_as_longlong(v); }
-
-// One pair (i, partner j at x, y, z of type tj) for the lane's ion: whether it is inside
-// r_cut (and both ions exist), and its force times the separation and energy.
-// 1/sqrt(x) for x in the range of squared pair distances (normal FP32 numbers): an FP32
-// seed (relative error below 2^-22) refined by two Newton-Raphson steps for x^(-1/2),
-// y <- y (3/2 - x y^2 / 2), each of which squares the relative error, so the result is
-// within a few ulp of the FP64 value.
+// 1/sqrt(x) for x in the range of squared pair distances (normal numbers): the hardware's
+// FP64 seed (rsqrt.approx.ftz.f64, from the upper 32 bits: relative error e below 2^-19) and
+// one third-order step y (1 + d / 2 + 3 d^2 / 8), d = 1 - x y^2, which leaves 5 e^3 / 2 < 2^-55.
 __device__ __forceinline__ double rsqrt_nr(double x) {
-    double y = (double)rsqrtf((float)x);
-    const double h = 0.5 * x;
-    y = y * fma(-h * y, y, 1.5);
-    y = y * fma(-h * y, y, 1.5);
-    return y;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double d = fma(-x * y, y, 1.0);
+    return fma(y * d, fma(d, 0.375, 0.5), y);
+}
+
+// x minus the nearest multiple of L: adding and subtracting 1.5 2^52 rounds to an integer.
+__device__ __forceinline__ double nearest_image(double x, double L, double invL) {
+    constexpr double kRound = 6755399441055744.0;
+    return fma(-L, fma(x, invL, kRound) - kRound, x);
 }
 
 struct PairSep {
     double dx, dy, dz, r2;
-    bool in;
 };
-__device__ __forceinline__ PairSep pair_sep(double L, double invL, double rc2, double xi, double yi, double zi, int ti,
-                                            double xj, double yj, double zj, int tj) {
+__device__ __forceinline__ PairSep pair_sep(double L, double invL, double xi, double yi, double zi, double xj, double yj,
+                                            double zj) {
     PairSep p;
-    p.dx = xi - xj;
-    p.dy = yi - yj;
-    p.dz = zi - zj;
-    p.dx -= L * round(p.dx * invL);
-    p.dy -= L * round(p.dy * invL);
-    p.dz -= L * round(p.dz * invL);
+    p.dx = nearest_image(xi - xj, L, invL);
+    p.dy = nearest_image(yi - yj, L, invL);
+    p.dz = nearest_image(zi - zj, L, invL);
     p.r2 = p.dx * p.dx + p.dy * p.dy + p.dz * p.dz;
-    p.in = ti >= 0 && tj >= 0 && p.r2 <= rc2;
     return p;
 }
-template <int POT>
-__device__ __forceinline__ void pair_force(const double* tab, int ntyp, double rc2, int ti, int tj, const PairSep& p,
-                                           double& ax, double& ay, double& az, double& vm) {
-    const double r2s = p.in ? p.r2 : rc2;  // a harmless value for lanes whose pair is not taken
-    double fr;
-    pair_terms<POT>(tab + kTfTabStride * ((p.in ? ti : 0) * ntyp + (p.in ? tj : 0)), r2s, rsqrt_nr(r2s), fr, vm);
-    ax = fr * p.dx;
-    ay = fr * p.dy;
-    az = fr * p.dz;
-}
-template <int POT>
-__device__ __forceinline__ bool pair_eval(const double* tab, int ntyp, double L, double invL, double rc2, double xi,
-                                          double yi, double zi, int ti, double xj, double yj, double zj, int tj,
-                                          double& ax, double& ay, double& az, double& vm) {
-    const PairSep p = pair_sep(L, invL, rc2, xi, yi, zi, ti, xj, yj, zj, tj);
-    pair_force<POT>(tab, ntyp, rc2, ti, tj, p, ax, ay, az, vm);
-    return p.in;
+// The exponential of TF: negligible beyond exp_limit for every type pair (tf_exp_r2_limit).
+// Apart from pair_terms, so that no branch stands between the two ions' other terms.
+__device__ __forceinline__ void pair_exp(const double2* t, double exp_limit, double r2, double ir, double& fr, double& vm) {
+    if (r2 < exp_limit) {
+        const double2 e = t[2];
+        const double ex = e.x * exp(e.y * (t[3].x - r2 * ir));
+        fr += e.y * ex * ir;
+        vm += ex;
+    }
 }
 
 template <int POT>
 __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
-    extern __shared__ double sm[];
-    double* tab = sm;                              // [64][kTfTabStride]
-    double* ipos = tab + kTfTab;                   // [4][256]: x, y, z, type (structure of arrays)
-    double* jpos = ipos + kTfSb * 32 * 4;          // [4][256]
-    double* fjw = jpos + kTfSb * 32 * 4;           // [8 warps][8 J blocks][3][32]
-    constexpr int NQ = kTfSb * 32;
+    extern __shared__ __align__(16) double sm[];
+    const int SB = P.tf_sb, NQ = SB * 32;
+    // the warps of an I pair: jparts of its J blocks, sparts of a block's 32 steps
+    const int ni = SB / 2, nj = tf_nj(SB), jparts = SB / nj, sparts = kTfWarps / ni / jparts;
+    double2* tab = reinterpret_cast<double2*>(sm);      // [65][kTfRow]
+    double* ipos = sm + 2 * kTfTab;                     // [SB][3][32]
+    double* jpos = ipos + NQ * 3;                       // [SB][3][32]
+    double* fjw = jpos + NQ * 3;                        // [8 warps][nj][3][32]
+    double* fiw = fjw + kTfWarps * nj * 96;             // [8 warps][2][3][32]
+    int* irow = reinterpret_cast<int*>(fiw + kTfWarps * 192);  // [SB][32]: first row of the ion's type
+    int* jrow = irow + NQ;                              // [SB][32]: row of the ion's type within it
     const int st = bx;
     const int SI = P.tf_st[2 * st], SJ = P.tf_st[2 * st + 1];
     const bool diag = SI == SJ;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wi = w % ni, part = w / ni, jp = part % jparts, sp = part / jparts;
+    const int t0 = jp * nj, s0 = sp * (32 / sparts), s1 = s0 + 32 / sparts;
     const int np = P.np, nblk = (np + 31) / 32, ntyp = P.ntyp;
     const double L = P.L, invL = 1.0 / L, rc2 = P.rcut * P.rcut;
+    const int rc2hi = __double2hiint(rc2);
     const double prune2 = rc2 * (1.0 + 1e-9);
     const bool prune = P.flags[1] == 0;
 
-    for (int x = threadIdx.x; x < ntyp * ntyp * kPairConsts; x += blockDim.x)
-        tab[(x / kPairConsts) * kTfTabStride + x % kPairConsts] = P.tab[x];
-    for (int q = threadIdx.x; q < NQ; q += blockDim.x) {
-        const int gi = SI * NQ + q, gj = SJ * NQ + q;
-        const bool vi = gi < np, vj = gj < np;
-        ipos[q] = vi ? P.spos[3 * gi] : 0.0;
-        ipos[NQ + q] = vi ? P.spos[3 * gi + 1] : 0.0;
-        ipos[2 * NQ + q] = vi ? P.spos[3 * gi + 2] : 0.0;
-        ipos[3 * NQ + q] = type_bits(vi ? P.stype[gi] : -1);
-        jpos[q] = vj ? P.spos[3 * gj] : 0.0;
-        jpos[NQ + q] = vj ? P.spos[3 * gj + 1] : 0.0;
-        jpos[2 * NQ + q] = vj ? P.spos[3 * gj + 2] : 0.0;
-        jpos[3 * NQ + q] = type_bits(vj ? P.stype[gj] : -1);
+    for (int x = threadIdx.x; x < ntyp * ntyp * kPairConsts; x += blockDim.x) {
+        const int c = x % kPairConsts, src = POT == POT_TF ? (0x74106532 >> (4 * c)) & 15 : c;
+        sm[(x / kPairConsts) * 2 * kTfRow + c] = P.tab[x - c + src];
     }
-    for (int x = threadIdx.x; x < kTfSb * kTfSb * 32 * 3; x += blockDim.x) fjw[x] = 0.0;
+    if (threadIdx.x < 2 * kTfRow) sm[2 * kTfZero + threadIdx.x] = 0.0;
+    for (int q = threadIdx.x; q < NQ; q += blockDim.x) {
+        const int gi = SI * NQ + q, gj = SJ * NQ + q, o = (q >> 5) * 96 + (q & 31);
+        const bool vi = gi < np, vj = gj < np;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            ipos[o + 32 * d] = vi ? P.spos[3 * gi + d] : 0.0;
+            jpos[o + 32 * d] = vj ? P.spos[3 * gj + d] : 0.0;
+        }
+        irow[q] = vi ? P.stype[gi] * ntyp * kTfRow : 0;
+        jrow[q] = vj ? P.stype[gj] * kTfRow : 0;
+    }
+    for (int x = threadIdx.x; x < kTfWarps * nj * 96; x += blockDim.x) fjw[x] = 0.0;
     __syncthreads();
+    double exp_limit = 0.0;
+    if (POT == POT_TF)
+        for (int x = 0; x < ntyp * ntyp; x++) exp_limit = fmax(exp_limit, tab[x * kTfRow + 3].y);
 
-    double fx = 0.0, fy = 0.0, fz = 0.0, e_acc = 0.0;
-    const int I = SI * kTfSb + w;
-    if (I < nblk) {
-        const int me = w * 32 + lane;
-        const double xi = ipos[me], yi = ipos[NQ + me], zi = ipos[2 * NQ + me];
-        const int ti = type_of(ipos[3 * NQ + me]);  // -1: no ion in this lane
-        const double* bI = P.tf_box + 6 * I;
-        for (int t = 0; t < kTfSb; t++) {
-            const int d = (t - w) & (kTfSb - 1);
-            if (diag && (d > kTfSb / 2 || (d == kTfSb / 2 && w >= kTfSb / 2))) continue;
-            const int J = SJ * kTfSb + t;
-            if (J >= nblk) continue;
-            const bool self = diag && d == 0;
-            if (prune && !self) {
-                const double* bJ = P.tf_box + 6 * J;
+    double fxa = 0.0, fya = 0.0, fza = 0.0, fxb = 0.0, fyb = 0.0, fzb = 0.0, e_acc = 0.0;
+    const int ba = 2 * wi, bb = ba + 1, Ia = SI * SB + ba, Ib = Ia + 1;
+    if (Ia < nblk) {
+        const double *pa = ipos + ba * 96 + lane, *pb = pa + 96;
+        const double xa = pa[0], ya = pa[32], za = pa[64], xb = pb[0], yb = pb[32], zb = pb[64];
+        const int rowa = irow[ba * 32 + lane], rowb = irow[bb * 32 + lane];
+        const bool va = Ia * 32 + lane < np, vb = Ib * 32 + lane < np;
+        // whether block I (its index bi in SI) is paired with J block t (J), and how: 0 not, 1
+        // every pair, 2 the block with itself
+        auto mode_of = [&](int I, int bi, int J, int t) {
+            if (I >= nblk || J >= nblk) return 0;
+            if (diag) {
+                const int d = (t - bi) & (SB - 1);
+                if (d == 0) return 2;
+                if (d > SB / 2 || (d == SB / 2 && bi >= SB / 2)) return 0;
+            }
+            if (prune) {
+                const double *bI = P.tf_box + 6 * I, *bJ = P.tf_box + 6 * J;
                 const double gx = axis_gap(bI[0], bI[3], bJ[0], bJ[3] - bJ[0], L);
                 const double gy = axis_gap(bI[1], bI[4], bJ[1], bJ[4] - bJ[1], L);
                 const double gz = axis_gap(bI[2], bI[5], bJ[2], bJ[5] - bJ[2], L);
-                if (gx * gx + gy * gy + gz * gz > prune2) continue;
+                if (gx * gx + gy * gy + gz * gz > prune2) return 0;
             }
-            const double* jx = jpos + t * 32;
-            const double* jy = jx + NQ;
-            const double* jz = jx + 2 * NQ;
-            const double* jt = jx + 3 * NQ;
-            double* fjx = fjw + (w * kTfSb + t) * 3 * 32;
-            double* fjy = fjx + 32;
-            double* fjz = fjx + 64;
-            if (self) {
-                // partners (l + s) mod 32 for s = 1..16, the last step by half the lanes, so
-                // every pair inside the block comes once
-                for (int s = 1; s <= 16; s++) {
+            return 1;
+        };
+        for (int t = t0; t < t0 + nj; t++) {
+            const int J = SJ * SB + t;
+            const int ma = mode_of(Ia, ba, J, t), mb = mode_of(Ib, bb, J, t);
+            if ((ma | mb) == 0) continue;
+            const double* jx = jpos + t * 96;
+            const int* jr = jrow + t * 32;
+            double* fj = fjw + (w * nj + t - t0) * 96;
+            const int left = np - J * 32;  // ions of block J, if fewer than 32
+            // all: every ion of the three blocks is there and every pair is taken
+            auto steps = [&](auto all) {
+                for (int s = s0; s < s1; s++) {
                     const int jj = (lane + s) & 31;
-                    double ax, ay, az, vm;
-                    const bool in = pair_eval<POT>(tab, ntyp, L, invL, rc2, xi, yi, zi, ti, jx[jj], jy[jj], jz[jj],
-                                                   type_of(jt[jj]), ax, ay, az, vm);
-                    if (in && !(s == 16 && lane >= 16)) {
-                        fx += ax;
-                        fy += ay;
-                        fz += az;
-                        fjx[jj] -= ax;
-                        fjy[jj] -= ay;
-                        fjz[jj] -= az;
-                        e_acc += vm;
+                    const double xj = jx[jj], yj = jx[32 + jj], zj = jx[64 + jj];
+                    const int row = jr[jj];
+                    const PairSep a = pair_sep(L, invL, xa, ya, za, xj, yj, zj);
+                    const PairSep b = pair_sep(L, invL, xb, yb, zb, xj, yj, zj);
+                    bool ina = a.r2 <= rc2, inb = b.r2 <= rc2;
+                    if (!all.value) {
+                        // a block with itself: each pair once
+                        const bool half = s >= 1 && (s < 16 || (s == 16 && lane < 16)), vj = jj < left;
+                        ina = ina && va && vj && (ma == 1 || (ma == 2 && half));
+                        inb = inb && vb && vj && (mb == 1 || (mb == 2 && half));
                     }
+                    // steps with no pair inside r_cut leave the terms out
+                    if (!__any_sync(0xffffffffu, ina || inb)) continue;
+                    // a pair that is not taken reads the row of zeros at a harmless distance (the
+                    // upper word of r_cut^2): its force and energy come out as zero
+                    const double2 *ra = tab + (ina ? rowa + row : kTfZero), *rb = tab + (inb ? rowb + row : kTfZero);
+                    const double r2a = __hiloint2double(ina ? __double2hiint(a.r2) : rc2hi, __double2loint(a.r2));
+                    const double r2b = __hiloint2double(inb ? __double2hiint(b.r2) : rc2hi, __double2loint(b.r2));
+                    const double ira = rsqrt_nr(r2a), irb = rsqrt_nr(r2b);
+                    double fa, ea, fb, eb;
+                    pair_terms<POT>(ra, r2a, ira, fa, ea);
+                    pair_terms<POT>(rb, r2b, irb, fb, eb);
+                    if (POT == POT_TF) {
+                        pair_exp(ra, exp_limit, r2a, ira, fa, ea);
+                        pair_exp(rb, exp_limit, r2b, irb, fb, eb);
+                    }
+                    fxa = fma(fa, a.dx, fxa);
+                    fya = fma(fa, a.dy, fya);
+                    fza = fma(fa, a.dz, fza);
+                    fxb = fma(fb, b.dx, fxb);
+                    fyb = fma(fb, b.dy, fyb);
+                    fzb = fma(fb, b.dz, fzb);
+                    fj[jj] = fma(-fa, a.dx, fma(-fb, b.dx, fj[jj]));
+                    fj[32 + jj] = fma(-fa, a.dy, fma(-fb, b.dy, fj[32 + jj]));
+                    fj[64 + jj] = fma(-fa, a.dz, fma(-fb, b.dz, fj[64 + jj]));
+                    e_acc += ea + eb;
                     __syncwarp();
                 }
-                continue;
-            }
-            // two partners per step, (l + s) and (l + s + 16) mod 32, as two independent
-            // chains; their reactions go in one after the other (each a permutation of the
-            // 32 entries)
-            for (int s = 0; s < 16; s++) {
-                const int ja = (lane + s) & 31, jb = (lane + s + 16) & 31;
-                double ax, ay, az, va, bx, by, bz, vb;
-                const int tja = type_of(jt[ja]), tjb = type_of(jt[jb]);
-                const PairSep pa = pair_sep(L, invL, rc2, xi, yi, zi, ti, jx[ja], jy[ja], jz[ja], tja);
-                const PairSep pb = pair_sep(L, invL, rc2, xi, yi, zi, ti, jx[jb], jy[jb], jz[jb], tjb);
-                if (!__any_sync(0xffffffffu, pa.in || pb.in)) continue;  // no pair of this step inside r_cut
-                pair_force<POT>(tab, ntyp, rc2, ti, tja, pa, ax, ay, az, va);
-                pair_force<POT>(tab, ntyp, rc2, ti, tjb, pb, bx, by, bz, vb);
-                const bool ina = pa.in, inb = pb.in;
-                if (ina) {
-                    fx += ax;
-                    fy += ay;
-                    fz += az;
-                    fjx[ja] -= ax;
-                    fjy[ja] -= ay;
-                    fjz[ja] -= az;
-                    e_acc += va;
-                }
-                __syncwarp();
-                if (inb) {
-                    fx += bx;
-                    fy += by;
-                    fz += bz;
-                    fjx[jb] -= bx;
-                    fjy[jb] -= by;
-                    fjz[jb] -= bz;
-                    e_acc += vb;
-                }
-                __syncwarp();
-            }
+            };
+            if (ma == 1 && mb == 1 && left >= 32 && Ib * 32 + 32 <= np)
+                steps(std::true_type());
+            else
+                steps(std::false_type());
         }
     }
-    // I side: this warp's block; J side: the warps' arrays summed in warp order
-    double* out = P.fpart + (size_t)st * 2 * kTfSb * 32 * 3;
-    if (I < nblk) {
-        double* o = out + (w * 32 + lane) * 3;
-        o[0] = fx;
-        o[1] = fy;
-        o[2] = fz;
-    }
-    __shared__ double esh[kTfSb];
+    // I and J sides: the warps' partials summed in warp order
+    double* out = P.fpart + (size_t)st * 2 * SB * 96;
+    double* fi = fiw + w * 192 + lane;
+    fi[0] = fxa;
+    fi[32] = fya;
+    fi[64] = fza;
+    fi[96] = fxb;
+    fi[128] = fyb;
+    fi[160] = fzb;
+    __shared__ double esh[kTfWarps];
     e_acc = warp_sum(e_acc);
     if (lane == 0) esh[w] = e_acc;
     __syncthreads();
-    for (int x = threadIdx.x; x < kTfSb * 32 * 3; x += blockDim.x) {
-        const int t = x / 96, jj = (x / 3) % 32, dd = x % 3;  // out layout [J block][32][3]
-        const int y = (t * 3 + dd) * 32 + jj;                  // warp arrays [J block][3][32]
+    for (int x = threadIdx.x; x < SB * 96; x += blockDim.x) {
+        const int t = x / 96, jj = (x / 3) % 32, dd = x % 3;  // out layout [block][32][3]
         double v = 0.0;
-        for (int q = 0; q < kTfSb; q++) v += fjw[q * kTfSb * 32 * 3 + y];
-        out[kTfSb * 32 * 3 + x] = v;
+        for (int q = t / 2; q < kTfWarps; q += ni) v += fiw[q * 192 + (t & 1) * 96 + dd * 32 + jj];
+        out[x] = v;
+        const int owner = t / nj, y = ((t - owner * nj) * 3 + dd) * 32 + jj;  // warp arrays [J block][3][32]
+        v = 0.0;
+        for (int q = 0; q < kTfWarps; q++)
+            if ((q / ni) % jparts == owner) v += fjw[q * nj * 96 + y];
+        out[SB * 96 + x] = v;
     }
     if (threadIdx.x == 0) {
         double e = 0.0;
-        for (int q = 0; q < kTfSb; q++) e += esh[q];
+        for (int q = 0; q < kTfWarps; q++) e += esh[q];
         P.epart[st] = e;
     }
 }
 template <int POT>
-__global__ void __launch_bounds__(kTfThreads, 3) k_tf(ParticleDev P) { k_tf_body<POT>(P, blockIdx.x); }
+__global__ void __launch_bounds__(kTfThreads, kTfResident) k_tf(ParticleDev P) { k_tf_body<POT>(P, blockIdx.x); }
 
-// Each ion's force: its super-tile partials in list order, scattered back to ion order.
-// A warp per block of 32 cell-ordered ions: the block's list is walked once for all 32
-// lanes (one ion each), whose partials lie side by side.
-__device__ __forceinline__ void k_tf_gather_body(const ParticleDev& P, int bx) {
-    const int b = (int)((bx * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (b >= (P.np + 31) / 32) return;
+// Each ion's force: its super-tile partials in list order, scattered back to ion order. A CTA
+// of four warps per block of 32 cell-ordered ions: each warp sums a quarter of the block's
+// list for all 32 lanes (one ion each, their partials side by side), and the quarters are
+// added in order. (One warp per block was a chain of up to 60 loads: 12 us where SB is small.)
+constexpr int kTfGather = 4;
+__device__ __forceinline__ void k_tf_gather_body(const ParticleDev& P, int b) {
+    __shared__ double part[kTfGather][96];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double f[3] = {0.0, 0.0, 0.0};
-    const int e1 = P.tf_gstart[b + 1];
-#pragma unroll 4
-    for (int e = P.tf_gstart[b]; e < e1; e++) {
+    const int g0 = P.tf_gstart[b], len = P.tf_gstart[b + 1] - g0;
+    const int e1 = g0 + len * (w + 1) / kTfGather;
+#pragma unroll 8
+    for (int e = g0 + len * w / kTfGather; e < e1; e++) {
         const int ent = P.tf_gent[e];
         const int st = ent >> 4, side = (ent >> 3) & 1, slot = ent & 7;
-        const double* o = P.fpart + (((size_t)st * 2 + side) * kTfSb + slot) * 32 * 3 + lane * 3;
+        const double* o = P.fpart + (((size_t)st * 2 + side) * P.tf_sb + slot) * 32 * 3 + lane * 3;
         f[0] += o[0];
         f[1] += o[1];
         f[2] += o[2];
     }
+#pragma unroll
+    for (int d = 0; d < 3; d++) part[w][d * 32 + lane] = f[d];
+    __syncthreads();
     const int s = b * 32 + lane;
-    if (s >= P.np) return;
+    if (w != 0 || s >= P.np) return;
     const int p = P.cell_ions[s];
-    P.fn[3 * p] = f[0];
-    P.fn[3 * p + 1] = f[1];
-    P.fn[3 * p + 2] = f[2];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        double v = part[0][d * 32 + lane];
+        for (int q = 1; q < kTfGather; q++) v += part[q][d * 32 + lane];
+        P.fn[3 * p + d] = v;
+    }
 }
 __global__ void k_tf_gather(ParticleDev P) { k_tf_gather_body(P, blockIdx.x); }
 
@@ -354,7 +385,12 @@ void tf_plan(ParticleDev& P) {
     dev_free(P.fpart);
     dev_free(P.epart);
     const int nblk = (P.np + 31) / 32 > 0 ? (P.np + 31) / 32 : 1;
-    const int nsb = (nblk + kTfSb - 1) / kTfSb;
+    int sb = kTfSbMax, nsb = (nblk + sb - 1) / sb;
+    while (sb > 2 && nsb * (nsb + 1) / 2 < kTfMinCtas) {
+        sb /= 2;
+        nsb = (nblk + sb - 1) / sb;
+    }
+    P.tf_sb = sb;
     std::vector<int> st;
     for (int si = 0; si < nsb; si++) {
         st.push_back(si);
@@ -369,8 +405,8 @@ void tf_plan(ParticleDev& P) {
     std::vector<std::vector<int>> lists(nblk);
     for (int k = 0; k < P.tf_nst; k++)
         for (int side = 0; side < 2; side++)
-            for (int slot = 0; slot < kTfSb; slot++) {
-                const int b = st[2 * k + side] * kTfSb + slot;
+            for (int slot = 0; slot < sb; slot++) {
+                const int b = st[2 * k + side] * sb + slot;
                 if (b < nblk) lists[b].push_back((k << 4) | (side << 3) | slot);
             }
     std::vector<int> gstart(nblk + 1, 0), gent;
@@ -387,7 +423,7 @@ void tf_plan(ParticleDev& P) {
     up((void**)&P.tf_gstart, gstart.data(), sizeof(int) * gstart.size());
     up((void**)&P.tf_gent, gent.data(), sizeof(int) * gent.size());
     P.tf_box = static_cast<double*>(dev_alloc(sizeof(double) * 6 * nblk));
-    P.fpart = static_cast<double*>(dev_alloc(sizeof(double) * (size_t)P.tf_nst * 2 * kTfSb * 32 * 3));
+    P.fpart = static_cast<double*>(dev_alloc(sizeof(double) * (size_t)P.tf_nst * 2 * sb * 32 * 3));
     P.epart = static_cast<double*>(dev_alloc(sizeof(double) * P.tf_nst));
     static unsigned long long attr_done = 0;  // devices whose kernels allow kTfSmem
     int dev = 0;
@@ -412,13 +448,13 @@ void tf_forces(ParticleDev& P, cudaStream_t s) {
     k_tf_boxes<<<(nblk * 32 + 255) / 256, 256, 0, s>>>(P);
     count_launch();
     if (P.pot == POT_LJ)
-        k_tf<POT_LJ><<<P.tf_nst, kTfThreads, kTfSmem, s>>>(P);
+        k_tf<POT_LJ><<<P.tf_nst, kTfThreads, tf_smem(P.tf_sb), s>>>(P);
     else if (P.pot == POT_SC)
-        k_tf<POT_SC><<<P.tf_nst, kTfThreads, kTfSmem, s>>>(P);
+        k_tf<POT_SC><<<P.tf_nst, kTfThreads, tf_smem(P.tf_sb), s>>>(P);
     else
-        k_tf<POT_TF><<<P.tf_nst, kTfThreads, kTfSmem, s>>>(P);
+        k_tf<POT_TF><<<P.tf_nst, kTfThreads, tf_smem(P.tf_sb), s>>>(P);
     count_launch();
-    k_tf_gather<<<(nblk * 32 + 127) / 128, 128, 0, s>>>(P);
+    k_tf_gather<<<nblk, kTfGather * 32, 0, s>>>(P);
     count_launch();
     k_tf_energy<<<1, 1024, 0, s>>>(P);
     MZB_CHECK(cudaGetLastError());
@@ -432,7 +468,7 @@ __global__ void __launch_bounds__(256) kt_tfbox(const StageArgs* __restrict__ A,
     table_run(A, start, nsys, [&](const StageArgs& a, int b) { k_tf_boxes_body(a.P, b); });
 }
 template <int POT>
-__global__ void __launch_bounds__(kTfThreads, 3) kt_tf(const StageArgs* __restrict__ A, const int* __restrict__ start,
+__global__ void __launch_bounds__(kTfThreads, kTfResident) kt_tf(const StageArgs* __restrict__ A, const int* __restrict__ start,
                                                        int nsys) {
     table_run(A, start, nsys, [&](const StageArgs& a, int b) { k_tf_body<POT>(a.P, b); });
 }

@@ -35,11 +35,13 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 }
 
 // Returns true once the barrier's phase with the given parity has completed, false if
-// the wall-clock limit expired first.
+// the wall-clock limit expired first. The timer is read only by waits that outlast kTmaPolls
+// polls (each suspends for a while in hardware): a read costs more than a landed slab's wait.
+constexpr int kTmaPolls = 16;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     const uint32_t a = smem_u32(bar);
-    const unsigned long long t0 = global_ns();
-    while (true) {
+    unsigned long long t0 = 0;
+    for (int polls = 0;; polls++) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -49,7 +51,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
             : "r"(a), "r"(parity)
             : "memory");
         if (done) return true;
-        if (global_ns() - t0 > kTmaWaitNs) return false;
+        if (polls < kTmaPolls) continue;
+        if (polls == kTmaPolls)
+            t0 = global_ns();
+        else if (global_ns() - t0 > kTmaWaitNs)
+            return false;
     }
 }
 

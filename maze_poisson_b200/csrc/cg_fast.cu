@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncthreads();
         if (abort_sh) {
             ok = false;
-            atomicOr(&a.bar->err, 1u);
+            mono_fail(a.bar);
             break;
         }
         // phase B reads own points only: its first slabs are fetched while alpha is reduced
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncthreads();
         if (abort_sh) {
             ok = false;
-            atomicOr(&a.bar->err, 1u);
+            mono_fail(a.bar);
             break;
         }
         stamp_it(a, iter, 2);

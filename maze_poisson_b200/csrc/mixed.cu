@@ -80,28 +80,7 @@ __device__ __forceinline__ bool team_sync(const Team& t, unsigned int& epoch) {
         return true;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&t.bar->count) : "memory");
-        const unsigned int target = (epoch + 1u) * (unsigned)t.nblk;
-        const unsigned long long t0 = global_ns();
-        unsigned int polls = 0;
-        while (ld_acquire_u32(&t.bar->count) < target) {
-            if ((++polls & 255u) == 0u) {
-                if (ld_relaxed_u32(&t.bar->err) != 0u) {
-                    ok = 0;
-                    break;
-                }
-                if (global_ns() - t0 > kBarrierTimeoutNs) {
-                    atomicOr(&t.bar->err, 1u);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        if (ok && ld_relaxed_u32(&t.bar->err) != 0u) ok = 0;
-        ok_sh = ok;
-    }
+    if (threadIdx.x == 0) ok_sh = mono_arrive_wait(t.bar, (epoch + 1u) * (unsigned)t.nblk);
     epoch++;
     __syncthreads();
     return ok_sh != 0;

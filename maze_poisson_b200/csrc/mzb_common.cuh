@@ -104,10 +104,10 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
 // a wall-clock limit read from %globaltimer: on expiry the waiter sets `err` and returns
 // false, so a lost block can never hang the GPU.
 // ------------------------------------------------------------------------------------
-struct GridBarrier {
+struct alignas(8) GridBarrier {
     unsigned int count;
     unsigned int gen;
-    unsigned int err;
+    unsigned int err;  // with pad: the word of the monotonic barrier (tma.cuh), which uses nothing else
     unsigned int pad;
 };
 

@@ -246,7 +246,7 @@ __device__ __forceinline__ bool block_total(double& v, bool any) {
 }
 
 // Sum of s and maximum of m over the grid through per-CTA partials and a grid barrier: the
-// way for values of any size (first use of a sum, fast_sum's overflow).
+// way for values of any size (first use of a sum, one that grew or shrank too much for fast_sum).
 struct Reduced {
     double sum, max;
     bool ok;
@@ -296,10 +296,14 @@ __device__ __noinline__ Reduced slow_reduce(const ResArgs& a, int slow_seq, doub
 // the arrivals, bits 40.. of `hi` the CTAs that raised `mark` and bits 48.. those whose value
 // does not fit (more than 512 times the previous sum, or not finite). Integer addition does
 // not depend on the order, the words are never cleared (each use subtracts the value after
-// the one before; two words alternate, so a word is read by all before it is used again),
-// and what is rounded away is below 2^-64 of the previous sum. The wait returns 0: the sum is
-// in res[0] and the marks in res[1]; 1: a value did not fit (all CTAs learn it); -1: it ran
-// out of time.
+// the one before; two words alternate, so a word is read by all before it is used again).
+// Up to 148 fractions rounded to 2^-48 leave an error below 2^-41.7 in a sum whose predecessor
+// stands at 2^22: less than FP64 rounds away itself unless the sum has shrunk by more than 2^11
+// (a smooth right-hand side can take it to 2^-100 in one iteration), and then it is taken
+// through the partials. The wait returns 0: the sum is in res[0] and the marks in res[1]; 1: a
+// value did not fit or the sum is too small (all CTAs read the same words); -1: it ran out of
+// time.
+constexpr long long kSmallestSum = 1 << 11;
 struct Posted {
     double inv_scale;
 };
@@ -345,9 +349,11 @@ __device__ __forceinline__ int fast_sum_wait(const ResArgs& a, int seq, const Po
     sh.lo[s] = x;
     sh.hi[s] = y;
     if (((dh >> 48) & 0xff) != 0) return 1;
-    const double H = (double)((long long)(dh & (((u64)1 << 40) - 1)) - (long long)(G << 31));
+    const long long whole = (long long)(dh & (((u64)1 << 40) - 1)) - (long long)(G << 31);
+    // the fractions add less than G + 1 to it
+    if ((u64)(whole + kSmallestSum + (long long)G) < (u64)(2 * kSmallestSum + (long long)G)) return 1;
     const double F = (double)(dl & (((u64)1 << 56) - 1)) * 0x1p-48;
-    sh.res[0] = (H + F) * posted.inv_scale;
+    sh.res[0] = ((double)whole + F) * posted.inv_scale;
     sh.res[1] = (double)((dh >> 40) & 0xff);
     return 0;
 }

@@ -9,6 +9,7 @@
 // in one file-scope __device__ array of fixed size below. That array exists in every
 // device that loads this library and stays allocated until the process exits.
 #include "engine.cuh"
+#include "resident.cuh"
 
 namespace mzb {
 namespace {
@@ -17,7 +18,8 @@ namespace {
 constexpr int kNoAllocMaxN = 64;
 constexpr long kNoAllocGrid = (long)kNoAllocMaxN * kNoAllocMaxN * kNoAllocMaxN;
 constexpr long kNoAllocPartials = 4096;  // doubles for the per-block reduction partials
-// r, p0, p1, Ap (n^3 each), partials, then barrier + result words: about 8.4 MB
+// r, p0, p1, Ap (n^3 each; or the resident kernel's halo area, at most 8.0 MB), partials, then
+// barrier + result words: about 8.4 MB
 constexpr long kNoAllocDoubles = 4 * kNoAllocGrid + kNoAllocPartials + 16;
 
 static __device__ __align__(256) double g_noalloc_work[kNoAllocDoubles];
@@ -114,8 +116,12 @@ extern "C" int mzb_conj_grad_noalloc(const double* b, const double* x0, double* 
     a.partials = w + 4 * kNoAllocGrid;
     a.bar = reinterpret_cast<GridBarrier*>(w + 4 * kNoAllocGrid + kNoAllocPartials);
     a.result = reinterpret_cast<int*>(w + 4 * kNoAllocGrid + kNoAllocPartials + 4);
+    // The resident kernel, as mzb_conj_grad takes for these sizes (the same bits); it needs none
+    // of r, p0, p1 and Ap, so its halo area takes their place. The streaming CG, made for grids
+    // above 128^3, takes 14.2 / 16.4 us an iteration at 48^3 / 64^3 where this takes 5.
+    if (resident_halo_bytes(n) <= 4 * kNoAllocGrid * sizeof(double)) a.halo = w;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!cg_fast_launch(a, s)) engine_launch(a, s);
+    if (!resident_cg_launch(a, s) && !cg_fast_launch(a, s)) engine_launch(a, s);
     int res[2] = {0, 0};
     cudaError_t e = cudaMemcpyAsync(res, a.result, sizeof(res), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

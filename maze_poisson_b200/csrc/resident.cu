@@ -1619,6 +1619,7 @@ bool resident_cg_launch(const EngineArgs& e, cudaStream_t stream) {
     else if (e.prog != PROG_CG && e.prog != PROG_INIT_FIELD && e.prog != PROG_LCG_UPDATE && e.prog != PROG_MAZE_LCG)
         return false;
     if (kind != PC_IMPLICIT && kind != PC_JACOBI) return false;
+    if ((uintptr_t)e.x & 15) return false;  // a caller's own buffer; x is written in pairs
     const Plan pl = make_plan(e.n, sm_count());
     if (!pl.Pi) return false;
     ResArgs a = common_args(e, pl);

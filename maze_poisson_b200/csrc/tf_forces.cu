@@ -29,10 +29,11 @@
 // issue 60 %): a pair loaded its partner, seven constants and the reaction, 34 wavefronts for
 // 40 FP64 instructions, and a 64-bit load costs an SM four times what an FP64 instruction
 // does. So one J ion serves two I ions, a pair beyond the exponential's range reads four
-// constants in two loads, and nothing goes through the conversion pipe: the nearest image by adding and subtracting 1.5 2^52, 1/r from the hardware's FP64
-// seed and one third-order step. Pairs that are not taken read a row of zeros instead of being
+// constants in two loads, and nothing goes through the conversion pipe: the nearest image by
+// adding and subtracting 1.5 2^52, 1/r from the hardware's FP64 approximation and two
+// Newton-Raphson steps. Pairs that are not taken read a row of zeros instead of being
 // selected out, and the exponential's branch follows both ions' other terms. At 16000 ions TF
-// 659 -> 553 us, LJ 569 -> 478 us: 84 instructions and 43 FP64 instructions a pair (104 and 43
+// 659 -> 559 us, LJ 569 -> 486 us: 84 instructions and 43 FP64 instructions a pair (104 and 43
 // with selects and single-ion lanes), FP64 pipe 60 %, issue 61 %; what is left is the latency of
 // 16 warps of two chains and the CTA's slowest warp.
 //
@@ -132,14 +133,18 @@ __device__ __forceinline__ void k_tf_boxes_body(const ParticleDev& P, int bx) {
 }
 __global__ void k_tf_boxes(ParticleDev P) { k_tf_boxes_body(P, blockIdx.x); }
 
-// 1/sqrt(x) for x in the range of squared pair distances (normal numbers): the hardware's
-// FP64 seed (rsqrt.approx.ftz.f64, from the upper 32 bits: relative error e below 2^-19) and
-// one third-order step y (1 + d / 2 + 3 d^2 / 8), d = 1 - x y^2, which leaves 5 e^3 / 2 < 2^-55.
-__device__ __forceinline__ double rsqrt_nr(double x) {
+// 1/sqrt(x) for x in the range of squared pair distances (normal numbers): two Newton-Raphson
+// steps for f(y) = 1/y^2 - x, y <- y + y (1/2 - x y^2 / 2), each of which squares the relative
+// error, from the hardware's FP64 approximation (the PTX instruction rsqrt.approx.ftz.f64; its
+// error is not counted on: the result is held to a few units in the last place by a test of
+// pair forces against 80-bit arithmetic). k_tf at 16000 ions: 559 us; with an FP32 seed, which
+// takes two conversions a pair, 578; with rsqrt() 594.
+__device__ __forceinline__ double inv_sqrt(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double d = fma(-x * y, y, 1.0);
-    return fma(y * d, fma(d, 0.375, 0.5), y);
+    const double h = 0.5 * x;
+    y = fma(y, fma(-h * y, y, 0.5), y);
+    return fma(y, fma(-h * y, y, 0.5), y);
 }
 
 // x minus the nearest multiple of L: adding and subtracting 1.5 2^52 rounds to an integer.
@@ -273,7 +278,7 @@ __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
                     const double2 *ra = tab + (ina ? rowa + row : kTfZero), *rb = tab + (inb ? rowb + row : kTfZero);
                     const double r2a = __hiloint2double(ina ? __double2hiint(a.r2) : rc2hi, __double2loint(a.r2));
                     const double r2b = __hiloint2double(inb ? __double2hiint(b.r2) : rc2hi, __double2loint(b.r2));
-                    const double ira = rsqrt_nr(r2a), irb = rsqrt_nr(r2b);
+                    const double ira = inv_sqrt(r2a), irb = inv_sqrt(r2b);
                     double fa, ea, fb, eb;
                     pair_terms<POT>(ra, r2a, ira, fa, ea);
                     pair_terms<POT>(rb, r2b, irb, fb, eb);

@@ -815,10 +815,18 @@ __device__ __forceinline__ void k_cell_sort_gather_body(const ParticleDev& P, in
     __syncwarp();
     for (int x = b + lane; x < e; x += 32) {
         const int p = P.cell_ions[x];
-        P.spos[3 * x] = P.pos[3 * p];
-        P.spos[3 * x + 1] = P.pos[3 * p + 1];
-        P.spos[3 * x + 2] = P.pos[3 * p + 2];
-        P.stype[x] = P.types[p];
+        // an ion that is nowhere (a coordinate not finite, or so large that a difference may not
+        // be) takes part in no pair: type -1 and a place that harms no arithmetic
+        double r[3];
+        bool there = true;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            r[d] = P.pos[3 * p + d];
+            there = there && fabs(r[d]) < 1e300;
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) P.spos[3 * x + d] = there ? r[d] : 0.0;
+        P.stype[x] = there ? P.types[p] : -1;
         P.srank[p] = x;
     }
 }

@@ -63,7 +63,7 @@ struct ParticleDev {
     int32_t* cell_ions = nullptr;    // [np]
     int32_t* srank = nullptr;        // [np] position of ion p in cell order
     double* spos = nullptr;          // [np][3] positions in cell order
-    int32_t* stype = nullptr;        // [np]
+    int32_t* stype = nullptr;        // [np] their types, -1 for an ion that takes part in no pair
     // pair-force plan (tf_forces.cu): super-tiles of tf_sb x tf_sb blocks of 32 cell-ordered ions
     int tf_sb = 0;                   // 8, 4 or 2
     int tf_nst = 0;                  // super-tiles (CTAs of the pair-force kernel)

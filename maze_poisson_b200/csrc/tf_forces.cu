@@ -206,6 +206,7 @@ __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
         sm[(x / kPairConsts) * 2 * kTfRow + c] = P.tab[x - c + src];
     }
     if (threadIdx.x < 2 * kTfRow) sm[2 * kTfZero + threadIdx.x] = 0.0;
+    bool absent = false;  // an ion of either super-block takes part in no pair (ParticleDev::stype)
     for (int q = threadIdx.x; q < NQ; q += blockDim.x) {
         const int gi = SI * NQ + q, gj = SJ * NQ + q, o = (q >> 5) * 96 + (q & 31);
         const bool vi = gi < np, vj = gj < np;
@@ -214,11 +215,13 @@ __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
             ipos[o + 32 * d] = vi ? P.spos[3 * gi + d] : 0.0;
             jpos[o + 32 * d] = vj ? P.spos[3 * gj + d] : 0.0;
         }
-        irow[q] = vi ? P.stype[gi] * ntyp * kTfRow : 0;
-        jrow[q] = vj ? P.stype[gj] * kTfRow : 0;
+        const int ti = vi ? P.stype[gi] : 0, tj = vj ? P.stype[gj] : 0;
+        irow[q] = ti * ntyp * kTfRow;
+        jrow[q] = tj * kTfRow;
+        absent = absent || ti < 0 || tj < 0;
     }
     for (int x = threadIdx.x; x < kTfWarps * nj * 96; x += blockDim.x) fjw[x] = 0.0;
-    __syncthreads();
+    absent = __syncthreads_or(absent);
     double exp_limit = 0.0;
     if (POT == POT_TF)
         for (int x = 0; x < ntyp * ntyp; x++) exp_limit = fmax(exp_limit, tab[x * kTfRow + 3].y);
@@ -229,7 +232,7 @@ __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
         const double *pa = ipos + ba * 96 + lane, *pb = pa + 96;
         const double xa = pa[0], ya = pa[32], za = pa[64], xb = pb[0], yb = pb[32], zb = pb[64];
         const int rowa = irow[ba * 32 + lane], rowb = irow[bb * 32 + lane];
-        const bool va = Ia * 32 + lane < np, vb = Ib * 32 + lane < np;
+        const bool va = Ia * 32 + lane < np && rowa >= 0, vb = Ib * 32 + lane < np && rowb >= 0;
         // whether block I (its index bi in SI) is paired with J block t (J), and how: 0 not, 1
         // every pair, 2 the block with itself
         auto mode_of = [&](int I, int bi, int J, int t) {
@@ -267,7 +270,7 @@ __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
                     bool ina = a.r2 <= rc2, inb = b.r2 <= rc2;
                     if (!all.value) {
                         // a block with itself: each pair once
-                        const bool half = s >= 1 && (s < 16 || (s == 16 && lane < 16)), vj = jj < left;
+                        const bool half = s >= 1 && (s < 16 || (s == 16 && lane < 16)), vj = jj < left && row >= 0;
                         ina = ina && va && vj && (ma == 1 || (ma == 2 && half));
                         inb = inb && vb && vj && (mb == 1 || (mb == 2 && half));
                     }
@@ -299,7 +302,7 @@ __device__ __forceinline__ void k_tf_body(const ParticleDev& P, int bx) {
                     __syncwarp();
                 }
             };
-            if (ma == 1 && mb == 1 && left >= 32 && Ib * 32 + 32 <= np)
+            if (ma == 1 && mb == 1 && left >= 32 && Ib * 32 + 32 <= np && !absent)
                 steps(std::true_type());
             else
                 steps(std::false_type());

@@ -2487,7 +2487,8 @@ int mzb_batch_autotune(const int* handles, int nsys, double* out) {
 }
 
 // Bytes of device memory one system of n^3 grid points and n_p ions holds with the
-// FP32+refine field solve (fields, multigrid levels, particle and pair-force arrays);
+// FP32+refine field solve (fields, multigrid levels, the resident kernels' work area, particle
+// and pair-force arrays);
 // the request loop admits jobs against an HBM budget with it.
 double mzb_system_footprint(int n, int n_p) {
     const double m = (double)n * n * n;
@@ -2497,11 +2498,14 @@ double mzb_system_footprint(int n, int n_p) {
     for (int l = 0; l < L; l++) levels += 3.0 * 4.0 * (double)sizes[l] * sizes[l] * sizes[l];
     levels += 8.0 * (double)(n / 2) * (n / 2) * (n / 4 + 1);  // half spectrum of an FFT-solved coarse level
     const double grid = 8.0 * m * 10.0;  // q, phi x3, y, r, p0, p1, Ap, tmp
-    const int nblk = (n_p + 31) / 32 > 0 ? (n_p + 31) / 32 : 1;
-    const double nsb = std::ceil(nblk / 8.0);
-    const double super_tiles = nsb * (std::floor(nsb / 2.0) + 1.0);  // pair-force CTAs
-    const double parts = (double)n_p * (8.0 * 3 * 7 + 4.0 * 8) + super_tiles * 2 * 8 * 32 * 3 * 8.0;
-    return grid + levels + parts + 64.0 * 1024 * 1024;
+    const TfShape t = tf_shape(n_p);
+    const double super_tiles = 0.5 * t.nsb * (t.nsb + 1.0);  // pair-force CTAs
+    // per ion: seven vectors, the lists, the spline weights (whether or not the scheme has them);
+    // per super-tile: force partials, gather entries, energy
+    const double parts = (double)n_p * (8.0 * 3 * 7 + 4.0 * 8 + 8.0 * 12) +
+                         super_tiles * (2.0 * t.sb * (32 * 3 * 8.0 + 4.0) + 16.0);
+    const double halo = (double)resident_halo_bytes(n);  // the bootstrap's FP64 solve
+    return grid + levels + parts + halo + 64.0 * 1024 * 1024;
 }
 
 }  // extern "C"

@@ -100,6 +100,11 @@ void field_forces(ParticleDev& P, const double* phi, int n, double h, cudaStream
 // Linked cells (counting sort, stable by ion index) + Tosi-Fumi forces into P.fn;
 // pair energy / 2 into red[1].
 void build_cells(ParticleDev& P, cudaStream_t s);
+// The pair-force kernel's division of np ions: blocks of 32, blocks per super-block, super-blocks.
+struct TfShape {
+    int nblk, sb, nsb;
+};
+TfShape tf_shape(int np);
 // Super-tile list, gather lists and partial buffers of the pair-force kernel for P.np.
 void tf_plan(ParticleDev& P);
 void tf_forces(ParticleDev& P, cudaStream_t s);

@@ -1511,15 +1511,19 @@ constexpr size_t kSmemBudget = 226 * 1024;
 // r and A p up to 16.
 constexpr int kMaxPairs = 16, kMaxPairsX = 10;
 
+// SMs of the current device, a B200's 148 where there is none (planners ask for sizes too).
 int sm_count() {
-    static int dev_of = -1, sms = 0;
-    int dev;
-    MZB_CHECK(cudaGetDevice(&dev));
-    if (dev != dev_of) {
-        MZB_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        dev_of = dev;
+    static thread_local int dev_of = -1, sms = 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) {
+        if (dev == dev_of) return sms;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
+            dev_of = dev;
+            return sms;
+        }
     }
-    return sms;
+    (void)cudaGetLastError();
+    return 148;
 }
 
 // The patches of an n^3 grid: the split of the n x n rows that leaves the fewest pairs to the

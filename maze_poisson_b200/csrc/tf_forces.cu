@@ -385,6 +385,18 @@ __device__ __forceinline__ void k_tf_energy_body(const ParticleDev& P, int bx) {
 }
 __global__ void k_tf_energy(ParticleDev P) { k_tf_energy_body(P, blockIdx.x); }
 
+TfShape tf_shape(int np) {
+    TfShape t;
+    t.nblk = (np + 31) / 32 > 0 ? (np + 31) / 32 : 1;
+    t.sb = kTfSbMax;
+    t.nsb = (t.nblk + t.sb - 1) / t.sb;
+    while (t.sb > 2 && t.nsb * (t.nsb + 1) / 2 < kTfMinCtas) {
+        t.sb /= 2;
+        t.nsb = (t.nblk + t.sb - 1) / t.sb;
+    }
+    return t;
+}
+
 void tf_plan(ParticleDev& P) {
     dev_free(P.tf_st);
     dev_free(P.tf_gstart);
@@ -392,12 +404,8 @@ void tf_plan(ParticleDev& P) {
     dev_free(P.tf_box);
     dev_free(P.fpart);
     dev_free(P.epart);
-    const int nblk = (P.np + 31) / 32 > 0 ? (P.np + 31) / 32 : 1;
-    int sb = kTfSbMax, nsb = (nblk + sb - 1) / sb;
-    while (sb > 2 && nsb * (nsb + 1) / 2 < kTfMinCtas) {
-        sb /= 2;
-        nsb = (nblk + sb - 1) / sb;
-    }
+    const TfShape shape = tf_shape(P.np);
+    const int nblk = shape.nblk, sb = shape.sb, nsb = shape.nsb;
     P.tf_sb = sb;
     std::vector<int> st;
     for (int si = 0; si < nsb; si++) {

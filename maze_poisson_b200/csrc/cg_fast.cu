@@ -59,12 +59,10 @@ struct CgFastArgs {
     double* partials;
     GridBarrier* bar;
     int* result;
-    unsigned long long* stamps;  // optional phase timestamps (block 0), see kStampIters
+    unsigned long long* stamps;  // optional phase timestamps (block 0), see stamp()
 };
 
 namespace {
-
-constexpr int kStampIters = 6;  // iterations whose phase boundaries are time-stamped
 
 constexpr int kThreads = 1024;
 constexpr int kProducer = kThreads - 32;  // the last warp issues the TMA loads, the others compute
@@ -162,14 +160,14 @@ __device__ bool reduce(double* s, double* mx, const CgFastArgs& a, unsigned& epo
     return ok;
 }
 
-// slots 0..3: set-up; 4 + 4 it + {0..3}: phase ends of iteration it < kStampIters;
+// slots 0..3: set-up; 4 + 4 it + {0..3}: phase ends of iteration it < kCgStampIters;
 // 40 + 2 e + {0, 1}: slab e of the first phase A (compute done, next stage landed)
 __device__ __forceinline__ void stamp(const CgFastArgs& a, int slot) {
     if (a.stamps != nullptr && blockIdx.x == 0 && threadIdx.x == 0 && slot < 96)
         a.stamps[slot] = global_ns();
 }
 __device__ __forceinline__ void stamp_it(const CgFastArgs& a, long iter, int k) {
-    if (iter < kStampIters) stamp(a, 4 + 4 * (int)iter + k);
+    if (iter < kCgStampIters) stamp(a, 4 + 4 * (int)iter + k);
 }
 
 // z(r): the direction increment of the preconditioned residual, exactly as the
@@ -629,8 +627,6 @@ bool encode_grid_map(CUtensorMap* map, const double* base, int n, int bx, int by
 }
 
 bool cg_fast_supported(int n) { return n % 16 == 0 && n >= 16 && n <= 256; }
-
-int cg_fast_stamp_slots() { return 4 + 4 * kStampIters; }
 
 namespace {
 

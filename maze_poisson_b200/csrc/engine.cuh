@@ -91,8 +91,11 @@ struct EngineArgs {
     double* partials;  // 2 sets x 8 values x gridDim.x
     GridBarrier* bar;
     int* result;       // [0] program return value, [1] engine status (0 ok)
-    unsigned long long* stamps;  // optional phase timestamps of the CG kernel (or null)
+    unsigned long long* stamps;  // optional phase timestamps of the CG kernels (96, or null)
 };
+
+// Iterations whose phase boundaries the CG kernels time-stamp.
+constexpr int kCgStampIters = 6;
 
 // Launch the engine for `a` on `stream` (cooperative; shapes chosen once per device).
 void engine_launch(const EngineArgs& a, cudaStream_t stream);
@@ -100,7 +103,6 @@ void engine_launch(const EngineArgs& a, cudaStream_t stream);
 // PROG_MAZE_LCG without MG) on the TMA-staged kernel of cg_fast.cu; false when the grid
 // size or device does not allow it (the caller then uses engine_launch).
 bool cg_fast_launch(const EngineArgs& a, cudaStream_t stream);
-int cg_fast_stamp_slots();
 // The inverse of the 7-point Laplacian of one 10^3 block with Dirichlet edges
 // (precond_blockjacobi.c:14-69), row-major 1000 x 1000, computed once on the host.
 const std::vector<double>& block_jacobi_inverse();

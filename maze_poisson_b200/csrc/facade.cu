@@ -383,7 +383,7 @@ void launch_solver(const EngineArgs& a, cudaStream_t stream) {
 // is reported and turned into -1 ("not converged").
 int run_engine(System& s, const EngineArgs& a) {
     MZB_CHECK(cudaEventRecord(s.ev0, s.stream));
-    // MZB_PHASE_TIMING=1: time-stamp the phases of the CG kernel and print them (debug aid)
+    // MZB_PHASE_TIMING=1: time-stamp the phases of the CG kernels and print them (debug aid)
     static const bool stamps_on = getenv("MZB_PHASE_TIMING") != nullptr;
     static unsigned long long* stamps_d = nullptr;
     EngineArgs b = a;
@@ -400,13 +400,13 @@ int run_engine(System& s, const EngineArgs& a) {
         if (h[0]) {
             fprintf(stderr, "[cg phases us] pre %.2f sync %.2f init %.2f |", (h[1] - h[0]) * 1e-3,
                     (h[2] - h[1]) * 1e-3, 0.0);
-            for (int it = 0; it + 1 < (cg_fast_stamp_slots() - 4) / 4; it++) {
+            for (int it = 0; it + 1 < kCgStampIters; it++) {
                 const unsigned long long* t = h + 4 + 4 * it;
                 if (!t[0] || !t[4]) break;
                 fprintf(stderr, " A %.2f redA %.2f B %.2f redB %.2f |", (t[0] - (it ? t[-1] : h[2])) * 1e-3,
                         (t[1] - t[0]) * 1e-3, (t[2] - t[1]) * 1e-3, (t[3] - t[2]) * 1e-3);
             }
-            fprintf(stderr, "\n[cg phase A slabs us: sync+issue, p_new, stencil]");
+            if (h[40]) fprintf(stderr, "\n[cg phase A slabs us: sync+issue, p_new, stencil]");  // cg_fast only
             for (int e = 0; e < 18 && h[40 + 3 * e]; e++) {
                 const unsigned long long prev = e ? h[39 + 3 * e] : h[2];
                 fprintf(stderr, " %.2f,%.2f,%.2f", (h[40 + 3 * e] - prev) * 1e-3, (h[41 + 3 * e] - h[40 + 3 * e]) * 1e-3,

@@ -621,6 +621,18 @@ __device__ __forceinline__ double rz_term(double r) {
     return r * r;
 }
 
+// Phase times (EngineArgs::stamps, a debug aid): slots 0 .. 2 the set-up, 4 + 4 it + {0 .. 3}
+// the ends of p and A p, their sum, the update, its sum, of iteration it < kCgStampIters.
+// Kernels of their own (TIMED): tested at run time in every phase they cost 3 % at 64^3.
+template <bool TIMED>
+__device__ __forceinline__ void stamp(const ResArgs& a, int slot) {
+    if (TIMED && (blockIdx.x | threadIdx.x) == 0) a.e.stamps[slot] = global_ns();
+}
+template <bool TIMED>
+__device__ __forceinline__ void stamp_it(const ResArgs& a, long iter, int k) {
+    if (TIMED && iter < kCgStampIters) stamp<true>(a, 4 + 4 * (int)iter + k);
+}
+
 // ------------------------------------------------------------------------------------
 // The iteration. On entry tensor memory holds the patch's residual (unit m at tr + 4 m) and
 // x (tx + 4 m, or the grid at xg); rv is <r, z(r)> and r0 = max |r| (COARSE). Slots past a
@@ -628,7 +640,7 @@ __device__ __forceinline__ double rz_term(double r) {
 // iteration at convergence or -1, cg_coarse the number of iterations
 // (library/src/plcg.c:28-238, multigrid.c:13-96, multigrid_pb.c:16-97).
 // ------------------------------------------------------------------------------------
-template <bool PB, int KIND, bool COARSE, int HL>
+template <bool PB, int KIND, bool COARSE, int HL, bool TIMED>
 __device__ __forceinline__ int iterate(const ResArgs& a, Ctl& c, const Patch& p, int units, double* P, uint32_t tr, uint32_t tap, uint32_t tx, double* xg,
                        const Coef& cf, double rv, double r0, double tol, long limit, bool& ok) {
     Shared& sh = shared_state();
@@ -773,6 +785,7 @@ __device__ __forceinline__ int iterate(const ResArgs& a, Ctl& c, const Patch& p,
                 }
             }
         }
+        stamp_it<TIMED>(a, iter, 0);
         int how = 1;
         if (fixed_point_ok(pap_prev)) {
             double v = pap;
@@ -796,6 +809,7 @@ __device__ __forceinline__ int iterate(const ResArgs& a, Ctl& c, const Patch& p,
         }
         pap_prev = pap;
         if (COARSE && fabs(pap) < 1e-300) return (int)iter;
+        stamp_it<TIMED>(a, iter, 1);
         const double alpha = rv / pap;
         // r += alpha A p; <r, z(r)>; |r|_inf against the stop; edge rows out
         c.step++;
@@ -829,6 +843,7 @@ __device__ __forceinline__ int iterate(const ResArgs& a, Ctl& c, const Patch& p,
                 __syncwarp();
             }
         }
+        stamp_it<TIMED>(a, iter, 2);
         // x += alpha p, which nothing waits for: done while the sum and the halo travel
         auto advance_x = [&]() {
             if (xg == nullptr) {
@@ -902,6 +917,7 @@ __device__ __forceinline__ int iterate(const ResArgs& a, Ctl& c, const Patch& p,
             ok = d.ok;
             if (!ok) return -1;
         }
+        stamp_it<TIMED>(a, iter, 3);
         rr_prev = rr;
         if (!above) return COARSE ? (int)iter + 1 : (int)iter;
         const double rnv = KIND == PC_IMPLICIT ? -rr / 6.0 : rr;
@@ -952,7 +968,7 @@ __device__ __noinline__ double mg_rhs(const EngineArgs& e, int i, int j, int k) 
 }
 
 // conj_grad and its callers. HL: pairs of a row per lane (1 up to n = 64, 2 up to 128).
-template <bool PB, int KIND, int HL>
+template <bool PB, int KIND, int HL, bool TIMED>
 __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_constant__ ResArgs a) {
     Shared& sh = shared_state();
     const EngineArgs& e = a.e;
@@ -980,6 +996,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_c
         cf.db = e.dg[0];
     }
 
+    stamp<TIMED>(a, 0);
     double acc = 0.0;
 #pragma unroll 1
     for (int m = 0; m < units; m++) {
@@ -1003,12 +1020,14 @@ __global__ void __launch_bounds__(kThreads, 1) resident_cg_kernel(const __grid_c
         if (xg == nullptr) tm_store(tx + 4 * m, x0);
     }
     tm_stored();
+    stamp<TIMED>(a, 1);
     const Reduced start = slow_reduce(a, c.slow_seq++, acc, 0.0);
+    stamp<TIMED>(a, 2);
     acc = start.sum;
     bool ok = start.ok;
     int result = -1;
     if (ok)
-        result = iterate<PB, KIND, false, HL>(a, c, p, units, smem + kStateDoubles, tr, tap, tx, xg, cf, KIND == PC_IMPLICIT ? -acc : acc, 0.0, e.tol,
+        result = iterate<PB, KIND, false, HL, TIMED>(a, c, p, units, smem + kStateDoubles, tr, tap, tx, xg, cf, KIND == PC_IMPLICIT ? -acc : acc, 0.0, e.tol,
                                           (long)n * n, ok);
     if (ok) {
 #pragma unroll 1
@@ -1324,8 +1343,8 @@ __device__ __noinline__ bool coarse_solve(const ResArgs& a, Ctl& ctl, uint32_t t
     const Reduced start = slow_reduce(a, c.slow_seq++, acc, top);
     bool ok = start.ok;
     if (ok && start.max != 0.0)
-        iterate<PB, KIND, true, 1>(a, c, p, units, smem + a.coarse_at, tm, tap, tx, nullptr, cf,
-                                   KIND == PC_IMPLICIT ? -start.sum : start.sum, start.max, 1e-5, 50, ok);
+        iterate<PB, KIND, true, 1, false>(a, c, p, units, smem + a.coarse_at, tm, tap, tx, nullptr, cf,
+                                          KIND == PC_IMPLICIT ? -start.sum : start.sum, start.max, 1e-5, 50, ok);
 #pragma unroll 1
     for (int m = 0; m < units; m++) {
         Cell t[1];
@@ -1576,11 +1595,11 @@ Plan make_plan(int n, int sms) {
     return e.plan;
 }
 
-template <int HL>
+template <int HL, bool TIMED>
 const void* pick_kernel(bool pb, int kind) {
-    if (pb) return (const void*)resident_cg_kernel<true, PC_IMPLICIT, HL>;
-    if (kind == PC_JACOBI) return (const void*)resident_cg_kernel<false, PC_JACOBI, HL>;
-    return (const void*)resident_cg_kernel<false, PC_IMPLICIT, HL>;
+    if (pb) return (const void*)resident_cg_kernel<true, PC_IMPLICIT, HL, TIMED>;
+    if (kind == PC_JACOBI) return (const void*)resident_cg_kernel<false, PC_JACOBI, HL, TIMED>;
+    return (const void*)resident_cg_kernel<false, PC_IMPLICIT, HL, TIMED>;
 }
 
 std::atomic<u64> g_launches{0};
@@ -1629,7 +1648,9 @@ bool resident_cg_launch(const EngineArgs& e, cudaStream_t stream) {
     ResArgs a = common_args(e, pl);
     a.smem_doubles = (int)(pl.smem / sizeof(double));
     a.x_tmem = pl.pairs <= kMaxPairsX ? 1 : 0;
-    const void* kf = e.n <= 64 ? pick_kernel<1>(e.pb, kind) : pick_kernel<2>(e.pb, kind);
+    const bool one = e.n <= 64, timed = e.stamps != nullptr;
+    const void* kf = one ? (timed ? pick_kernel<1, true> : pick_kernel<1, false>)(e.pb, kind)
+                         : (timed ? pick_kernel<2, true> : pick_kernel<2, false>)(e.pb, kind);
     launch(kf, a, stream);
     return true;
 }

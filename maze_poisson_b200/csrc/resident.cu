@@ -236,11 +236,8 @@ __device__ __forceinline__ bool block_total(double& v, bool any) {
     const bool r = __syncthreads_or(any);
     if (threadIdx.x < kWarps) {
         v = sh.sum[threadIdx.x];
-        // Any order of the warps is as good. Multigrid forces move by up to 1e-9 with the last bit
-        // of a start field; with this order the 128^3 melt's stay within 6e-10 of the oracle's.
 #pragma unroll
-        for (int o : {2, 1, 8, 4}) v += __shfl_xor_sync((1u << kWarps) - 1u, v, o);
-        static_assert(kWarps == 16, "the order above");
+        for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync((1u << kWarps) - 1u, v, o);
     }
     return r;
 }

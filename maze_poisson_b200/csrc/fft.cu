@@ -569,8 +569,9 @@ void solve_reg(const double* q, double* phi, double2* spec, const double2* W, co
 
 using RegSolver = void (*)(const double*, double*, double2*, const double2*, const double*, const double*, double,
                            cudaStream_t);
-// The sizes worked in registers: the products of two factors of 4 .. 18 nearest each other,
-// up to 256 (one that is missing here, or larger, takes the Stockham kernels).
+// The sizes worked in registers, as the product of two factors of 4 .. 18 nearest each other. The
+// others take the Stockham kernels, also the few that have such factors (16, 24, 81, 288,
+// 324): no workload here has them.
 RegSolver reg_solver(int n) {
     switch (n) {
     case 32: return solve_reg<8, 4>;

@@ -33,8 +33,8 @@
 // adding and subtracting 1.5 2^52, 1/r from the hardware's FP64 approximation and two
 // Newton-Raphson steps. Pairs that are not taken read a row of zeros instead of being
 // selected out, and the exponential's branch follows both ions' other terms. At 16000 ions TF
-// 659 -> 559 us, LJ 569 -> 486 us: 84 instructions and 43 FP64 instructions a pair (104 and 43
-// with selects and single-ion lanes), FP64 pipe 60 %, issue 61 %; what is left is the latency of
+// 659 -> 559 us, LJ 569 -> 486 us: 90 instructions, 40 of them FP64, for each of the N (N - 1) / 2
+// pairs (123 instructions before), FP64 pipe 62 %, issue 61 %; what is left is the latency of
 // 16 warps of two chains and the CTA's slowest warp.
 //
 // Determinism. Registers and warp arrays accumulate in step order; the warps' partials are

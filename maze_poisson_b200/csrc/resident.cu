@@ -345,14 +345,13 @@ __device__ __forceinline__ int fast_sum_wait(const ResArgs& a, int seq, const Po
     }
     sh.lo[s] = x;
     sh.hi[s] = y;
-    if (((dh >> 48) & 0xff) != 0) return 1;
     const long long whole = (long long)(dh & (((u64)1 << 40) - 1)) - (long long)(G << 31);
-    // the fractions add less than G + 1 to it
-    if ((u64)(whole + kSmallestSum + (long long)G) < (u64)(2 * kSmallestSum + (long long)G)) return 1;
     const double F = (double)(dl & (((u64)1 << 56) - 1)) * 0x1p-48;
     sh.res[0] = ((double)whole + F) * posted.inv_scale;
     sh.res[1] = (double)((dh >> 40) & 0xff);
-    return 0;
+    // the fractions add less than G + 1 to the whole part; no branch, all warps wait for this
+    const bool small = (u64)(whole + kSmallestSum + (long long)G) < (u64)(2 * kSmallestSum + (long long)G);
+    return (int)(small | (((dh >> 48) & 0xff) != 0));
 }
 __device__ __forceinline__ bool fixed_point_ok(double prev) {
     const int ex = (int)((__double_as_longlong(prev) >> 52) & 0x7ff);
